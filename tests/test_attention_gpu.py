@@ -200,3 +200,25 @@ def test_decode_rope_and_cache_update_in_one_launch(bw, dev, fused_qkv):
     untouched = torch.ones(L, dtype=torch.bool)
     untouched[pos] = False
     assert bool((kc[:, :, untouched.to(dev)] == 9.0).all()) and bool((vc[:, :, untouched.to(dev)] == 9.0).all())
+
+
+@pytest.mark.parametrize("S", [1, 127, 129, 385, 640])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_forward_maximum_rises_with_every_block(bw, dev, native_sdp, S, causal, dt):
+    """The scores grow along the keys, so the softmax's reference maximum is raised and the output rescaled in every
+    block of 128 keys, also in one that the first half of a block has already been computed for."""
+    torch.manual_seed(5)
+    q = torch.randn(1, S, 2, 128).abs().to(dt).transpose(1, 2)
+    ramp = (torch.arange(S) / 32.0).view(1, S, 1, 1) * 0.4
+    k = (torch.randn(1, S, 2, 128) * 0.1 + ramp).to(dt).transpose(1, 2)
+    v = torch.randn(1, S, 2, 128).to(dt).transpose(1, 2)
+    ref, _ = ref_attention(q, k, v, causal)
+    before = bw._C._native_sdp_forward_calls()
+    out = F.scaled_dot_product_attention(q.to(dev), k.to(dev), v.to(dev), is_causal=causal)
+    assert bw._C._native_sdp_forward_calls() == before + 1
+    # P is rounded to 16 bits before it multiplies V (|v| < 5): 5 * 2^-9 (bf16) or 5 * 2^-12 (fp16), plus the output's rounding
+    tol = 2e-2 if dt == torch.bfloat16 else 4e-3
+    assert (out.float().cpu() - ref).abs().max() < tol
+    bw.synchronize()
+    assert bw._C._gemm_status(False) == 0

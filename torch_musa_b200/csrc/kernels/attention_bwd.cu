@@ -58,9 +58,6 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const 
                ::"l"(map), "r"(smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
 }
-__device__ __forceinline__ void named_bar_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
 
 template <typename T>
 __global__ void __launch_bounds__(kBwdThreads, 1)

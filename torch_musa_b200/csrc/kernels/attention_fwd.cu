@@ -6,6 +6,7 @@
 #include "attention_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace b200k {
 namespace {
@@ -13,11 +14,14 @@ using namespace gemmdev;
 using namespace attndev;
 
 constexpr int AQ = 128, AK = 128, AD = 128;          // query rows per tile, keys per block, head dim
-constexpr int kTile = 128 * 128 * 2;                  // 32 KB: any of Q, K, V, P
-constexpr int kRing = 3;                              // K / V tiles in flight
-constexpr int kAttnSmem = 2 * kTile /*Q0,Q1*/ + kRing * kTile + 2 * kTile /*P0,P1*/ + 1024 + 256;
-constexpr int kAttnThreads = 320;                     // 2 softmax warpgroups, TMA warp, MMA warp
+constexpr int kTile = 128 * 128 * 2;                  // 32 KB: any of Q, K, V
+constexpr int kRing = 5;                              // K / V tiles in flight
+constexpr int kAttnSmem = 2 * kTile /*Q0,Q1*/ + kRing * kTile + 1024 + 256;
+constexpr int kAttnThreads = 384;                     // 2 softmax warpgroups; one with the TMA warp and the MMA warp
+constexpr int kSoftmaxRegs = 216, kOtherRegs = 72;    // after the split: a row of scores stays in registers
+constexpr int kLaunchRegs = (2 * kSoftmaxRegs + kOtherRegs + 2) / 3;   // what the launch has to bring for that split
 constexpr uint32_t kAttnTmemCols = 512;               // S0, S1, O0, O1
+constexpr int kFirstPart = 64;                        // keys of a block whose P is released before the rest is computed
 constexpr float kRescaleThreshold = 8.f;              // log2 domain: P stays below 2^8
 
 struct AttnParams {
@@ -37,14 +41,24 @@ struct AttnParams {
 
 // One CTA owns two adjacent 128-row query tiles of one (batch, head).  Per block of 128 keys and per tile t:
 //   S_t = Q_t K^T     tcgen05.mma M128 N128 K16 x 8 into TMEM (operands in 128B-swizzled shared memory);
-//   softmax           warpgroup t, one query row per thread: two passes over the row of S in TMEM (block maximum, then
-//                     P = exp2(S * scale - m) as bf16 into shared memory in the layout of an A operand);
-//   O_t += P_t V      tcgen05.mma accumulating in TMEM over all key blocks.
+//   softmax           warpgroup t, one query row per thread: the row of S comes into registers once, P = exp2(S * scale - m)
+//                     goes back as 16-bit pairs into TMEM over the columns of S, the block maximum is found on the side;
+//   O_t += P_t V      tcgen05.mma with A = P from TMEM, accumulating in TMEM over all key blocks.
+// P never touches shared memory: the M128 N128 products with both operands there already take all of its 128 bytes per
+// clock, and writing P there, fencing the async proxy and reading it back stood in the middle of the chain S -> softmax ->
+// P V.  One barrier per tile says "all products of this tile so far are done" (S of block j and, before it, P V of block
+// j - 1), so the softmax may overwrite S with P and rescale O without another wait.  What bounds the kernel now is that
+// chain: per block of 128 keys about 2700 clocks of softmax (two warpgroups share the special-function unit: 2048 clocks of
+// exponentials for both), 1050 of products and 500 of hand-over, while the tensor core has 2100 clocks of work for both
+// tiles.  Measured at 32 heads x 4096 x 128 bf16, before -> after: causal 174 -> 139 us (990 TFLOP/s), full 300 -> 255 us;
+// 32 heads x 16384 causal 1790 us (1230 TFLOP/s).  Tried and not kept: a quarter to a half of the exponentials as polynomials
+// on the FMA pipe (+2 to +10 % time), two warpgroups per tile (+11 %), S in halves of 64 keys issued ahead (+12 %: an N64
+// product is bound by reading A from shared memory).
 // The exponent's reference maximum m is only raised when the running maximum has grown by more than 2^8 ("lazy"
 // rescaling): then the warpgroup multiplies its rows of O in TMEM (tcgen05.ld / st) before it releases P.  That is rare
 // after the first blocks, so O normally never leaves TMEM until the epilogue.
-// The MMA warp alternates between the tiles (P V of tile 0, next S of tile 0, P V of tile 1, next S of tile 1), so one
-// tile's softmax runs while the tensor core works for the other; K and V tiles stream through a three-slot TMA ring.
+// The MMA warp alternates between the tiles (P V and next S of tile 0, then of tile 1), so one tile's softmax runs while
+// the tensor core works for the other; K and V tiles stream through a five-slot TMA ring.
 template <typename T>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -53,16 +67,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;                          // [2][kTile]
   uint8_t* sR = smem + 2 * kTile;              // [kRing][kTile]
-  uint8_t* sP = smem + (2 + kRing) * kTile;    // [2][kTile]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (4 + kRing) * kTile);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (2 + kRing) * kTile);
   uint64_t* q_full = bars;                     // [2]
   uint64_t* r_full = bars + 2;                 // [kRing]
   uint64_t* r_empty = bars + 2 + kRing;        // [kRing]  tcgen05.commit
-  uint64_t* s_full = bars + 2 + 2 * kRing;     // [2]      tcgen05.commit
-  uint64_t* s_free = s_full + 2;               // [2]      four softmax warps
-  uint64_t* p_ready = s_free + 2;              // [2]      four softmax warps
-  uint64_t* pv_done = p_ready + 2;             // [2]      tcgen05.commit
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+  uint64_t* mma_done = bars + 2 + 2 * kRing;   // [2]      tcgen05.commit: P V of block j - 1 and S of block j
+  uint64_t* p_ready = mma_done + 2;            // [2][2]   four softmax warps: first / second part of P of block j is in TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_ready + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -96,10 +107,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     *abort_flag = 0;
     for (int t = 0; t < 2; ++t) {
       mbar_init(&q_full[t], 1);
-      mbar_init(&s_full[t], 1);
-      mbar_init(&s_free[t], 4);
-      mbar_init(&p_ready[t], 4);
-      mbar_init(&pv_done[t], 1);
+      mbar_init(&mma_done[t], 1);
+      mbar_init(&p_ready[2 * t], 4);
+      mbar_init(&p_ready[2 * t + 1], 4);
     }
     for (int s = 0; s < kRing; ++s) {
       mbar_init(&r_full[s], 1);
@@ -119,93 +129,100 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 8) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      for (int t = 0; t < 2; ++t) {
-        if (nb[t] == 0) continue;
-        const int q0 = (2 * qp + t) * AQ;
-        mbar_expect_tx(&q_full[t], kTile);
-        tma_load_4d(sQ + t * kTile, &tmap_q, &q_full[t], 0, qoff + q0, h, bt);                 // d 0..63
-        tma_load_4d(sQ + t * kTile + kTile / 2, &tmap_q, &q_full[t], 64, qoff + q0, h, bt);    // d 64..127
+  if (warp >= 8) {
+    regs_dec<kOtherRegs>();
+    if (warp == 8) {
+      // ------------------------------------------------------------ TMA producer
+      if (lane == 0) {
+        for (int t = 0; t < 2; ++t) {
+          if (nb[t] == 0) continue;
+          const int q0 = (2 * qp + t) * AQ;
+          mbar_expect_tx(&q_full[t], kTile);
+          tma_load_4d(sQ + t * kTile, &tmap_q, &q_full[t], 0, qoff + q0, h, bt);                 // d 0..63
+          tma_load_4d(sQ + t * kTile + kTile / 2, &tmap_q, &q_full[t], 64, qoff + q0, h, bt);    // d 64..127
+        }
+        for (int n = 0; n < 2 * nbmax; ++n) {
+          const int st = n % kRing;
+          if (!mbar_wait(&r_empty[st], (uint32_t)(((n / kRing) & 1) ^ 1), abort_flag)) break;
+          mbar_expect_tx(&r_full[st], kTile);
+          const int k0 = (n >> 1) * AK;
+          const CUtensorMap* map = (n & 1) ? &tmap_v : &tmap_k;   // V is read as an MN-major B operand: same boxes
+          tma_load_4d(sR + st * kTile, map, &r_full[st], 0, koff + k0, hk, bt);
+          tma_load_4d(sR + st * kTile + kTile / 2, map, &r_full[st], 64, koff + k0, hk, bt);
+        }
       }
-      for (int n = 0; n < 2 * nbmax; ++n) {
-        const int st = n % kRing;
-        if (!mbar_wait(&r_empty[st], (uint32_t)(((n / kRing) & 1) ^ 1), abort_flag)) break;
-        mbar_expect_tx(&r_full[st], kTile);
-        const int k0 = (n >> 1) * AK;
-        const CUtensorMap* map = (n & 1) ? &tmap_v : &tmap_k;   // V is read as an MN-major B operand: same boxes
-        tma_load_4d(sR + st * kTile, map, &r_full[st], 0, koff + k0, hk, bt);
-        tma_load_4d(sR + st * kTile + kTile / 2, map, &r_full[st], 64, koff + k0, hk, bt);
-      }
-    }
-    __syncwarp();
-  } else if (warp == 9) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+      __syncwarp();
+    } else if (warp == 9) {
+      // ------------------------------------------------------------ MMA issuer (the whole warp waits, one lane issues)
       // instruction descriptors: fp32 accumulate, bf16/fp16 operands, M128 N128; S: both K-major; PV: B MN-major
-      const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-      const uint32_t idesc_o = idesc_s | (1u << 16);
-      bool ok = true;
-      auto ring_wait = [&](int n) { return mbar_wait(&r_full[n % kRing], (uint32_t)((n / kRing) & 1), abort_flag); };
+      constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+      constexpr uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+      constexpr uint32_t idesc_o = idesc_s | (1u << 16);
+      const bool leader = elect_one();
+      const uint64_t q_desc = make_desc(smem_u32(sQ), 16, 1024);             // K-major tiles; + (bytes >> 4) for an offset
+      const uint64_t k_desc = make_desc(smem_u32(sR), 16, 1024);
+      const uint64_t v_desc = make_desc(smem_u32(sR), kTile / 2, 1024);      // MN-major
+      auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
+      auto ring_wait = [&](int n) { return wait(&r_full[n % kRing], (uint32_t)((n / kRing) & 1)); };
       auto issue_s = [&](int t, int n) {     // S_t = Q_t K^T with K in ring item n
-        const uint32_t qa = smem_u32(sQ + t * kTile), ka = smem_u32(sR + (n % kRing) * kTile);
-#pragma unroll
+        const uint64_t qa = q_desc + (uint32_t)(t * (kTile >> 4)), ka = k_desc + (uint32_t)((n % kRing) * (kTile >> 4));
+  #pragma unroll
         for (int kk = 0; kk < AD / 16; ++kk) {
-          const uint32_t off = (uint32_t)(kk >> 2) * (kTile / 2) + (uint32_t)(kk & 3) * 32;   // 64-column atom, 32 B per k16
-          umma_f16(tmem_base + (uint32_t)(t * 128), make_desc(qa + off, 16, 1024), make_desc(ka + off, 16, 1024), idesc_s,
-                   kk != 0 ? 1u : 0u);
+          const uint32_t off = ((uint32_t)(kk >> 2) * (kTile / 2) + (uint32_t)(kk & 3) * 32) >> 4;   // 64-column atom, 32 B per k16
+          umma_f16(tmem_base + (uint32_t)(t * 128), qa + off, ka + off, idesc_s, kk != 0 ? 1u : 0u);
         }
-        umma_commit(&s_full[t]);
       };
-      auto issue_pv = [&](int t, int n, bool first) {   // O_t (+)= P_t V with V in ring item n
-        const uint32_t pa = smem_u32(sP + t * kTile), va = smem_u32(sR + (n % kRing) * kTile);
-#pragma unroll
-        for (int kk = 0; kk < AK / 16; ++kk) {
-          // A = P (K-major over keys): two 64-key atoms; B = V (MN-major): 16 key rows = 2048 B, next 64-wide d box 16 KB on
-          const uint32_t aoff = (uint32_t)(kk >> 2) * (kTile / 2) + (uint32_t)(kk & 3) * 32;
-          umma_f16(tmem_base + 256u + (uint32_t)(t * 128), make_desc(pa + aoff, 16, 1024),
-                   make_desc(va + (uint32_t)kk * 2048, kTile / 2, 1024), idesc_o, (first && kk == 0) ? 0u : 1u);
-        }
-        umma_commit(&pv_done[t]);
+      auto issue_pv = [&](int t, int n, bool first, int kk0, int kk1) {   // O_t (+)= P_t V with V in ring item n
+        const uint32_t pa = tmem_base + (uint32_t)(t * 128);
+        const uint64_t va = v_desc + (uint32_t)((n % kRing) * (kTile >> 4));
+  #pragma unroll
+        for (int kk = kk0; kk < kk1; ++kk)
+          // A = P in TMEM, 8 columns per 16 keys; B = V (MN-major): 16 key rows = 2048 B, next 64-wide d box 16 KB on
+          umma_f16_ts(tmem_base + 256u + (uint32_t)(t * 128), pa + (uint32_t)(kk * 8), va + (uint32_t)(kk * (2048 >> 4)), idesc_o,
+                      (first && kk == 0) ? 0u : 1u);
       };
+      bool ok = true;
       for (int t = 0; t < 2 && ok; ++t)
-        if (nb[t] > 0) ok = mbar_wait(&q_full[t], 0, abort_flag);
+        if (nb[t] > 0) ok = wait(&q_full[t], 0);
       if (ok && nbmax > 0) ok = ring_wait(0);
       if (ok && nbmax > 0) {
         tc_fence_after();
-        for (int t = 0; t < 2; ++t)
-          if (nb[t] > 0) issue_s(t, 0);
-        umma_commit(&r_empty[0]);
+        if (leader) {
+          for (int t = 0; t < 2; ++t)
+            if (nb[t] > 0) {
+              issue_s(t, 0);
+              umma_commit(&mma_done[t]);
+            }
+          umma_commit(&r_empty[0]);
+        }
       }
       for (int j = 0; j < nbmax && ok; ++j) {
         const int nv = 2 * j + 1, nk = 2 * j + 2;
         if (!ring_wait(nv)) { ok = false; break; }
-        bool k_ready = false;
-        for (int t = 0; t < 2 && ok; ++t) {
-          if (j < nb[t]) {
-            if (!mbar_wait(&p_ready[t], (uint32_t)(j & 1), abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            issue_pv(t, nv, j == 0);
-          }
-          if (j + 1 < nb[t]) {
-            if (!k_ready) {
-              if (!ring_wait(nk)) { ok = false; break; }
-              k_ready = true;
-            }
-            if (!mbar_wait(&s_free[t], (uint32_t)(j & 1), abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            issue_s(t, nk);
+        if (j + 1 < nbmax && !ring_wait(nk)) { ok = false; break; }
+        for (int t = 0; t < 2; ++t) {
+          if (j >= nb[t]) continue;
+          if (!wait(&p_ready[2 * t], (uint32_t)(j & 1))) { ok = false; break; }
+          tc_fence_after();
+          if (leader) issue_pv(t, nv, j == 0, 0, kFirstPart / 16);
+          if (!wait(&p_ready[2 * t + 1], (uint32_t)(j & 1))) { ok = false; break; }
+          tc_fence_after();
+          if (leader) {
+            issue_pv(t, nv, false, kFirstPart / 16, AK / 16);
+            if (j + 1 < nb[t]) issue_s(t, nk);     // over P of block j: the tensor core works in issue order
+            umma_commit(&mma_done[t]);
           }
         }
         if (!ok) break;
-        umma_commit(&r_empty[nv % kRing]);
-        if (j + 1 < nbmax) umma_commit(&r_empty[nk % kRing]);
+        if (leader) {
+          umma_commit(&r_empty[nv % kRing]);
+          if (j + 1 < nbmax) umma_commit(&r_empty[nk % kRing]);
+        }
       }
+      __syncwarp();
     }
-    __syncwarp();
   } else {
+    regs_inc<kSoftmaxRegs>();
     // ------------------------------------------------------------ softmax warpgroup t (warps 4t .. 4t+3)
     const int t = warp >> 2;
     const int qw = warp & 3;                 // TMEM lane quarter of this warp
@@ -214,7 +231,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const uint32_t lane_base = ((uint32_t)(qw * 32) << 16);
     const uint32_t s_addr = tmem_base + lane_base + (uint32_t)(t * 128);
     const uint32_t o_addr = tmem_base + lane_base + 256u + (uint32_t)(t * 128);
-    uint8_t* prow = sP + t * kTile + (size_t)r * 128;
     float m_ref = -INFINITY;                 // maximum the exponents refer to (raised lazily)
     float l_run = 0.f;
     bool ok = true;
@@ -225,7 +241,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       return __all_sync(0xffffffffu, w);
     };
     for (int j = 0; j < n_blocks; ++j) {
-      if (!wait_all(&s_full[t], (uint32_t)(j & 1))) { ok = false; break; }
+      if (!wait_all(&mma_done[t], (uint32_t)(j & 1))) { ok = false; break; }
       tc_fence_after();
       const int k0 = j * AK;
       // the row's visible keys: [0, lim)
@@ -233,111 +249,97 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (p.causal) lim = min(lim, qi - k0 + 1);
       lim = max(0, min(lim, AK));
       const bool full = __all_sync(0xffffffffu, lim == AK);
-      // pass 1: block maximum of the raw scores (the TMEM load of one 32-column chunk overlaps the work on the other)
-      float m_blk = -INFINITY;
-      {
-        uint32_t ra[32], rb[32];
-        auto chunk_max = [&](const uint32_t (&raw)[32], int c) {
-          if (full) {
+      // the whole row of scores in registers
+      uint32_t raw[4][32];
 #pragma unroll
-            for (int e = 0; e < 32; ++e) m_blk = fmaxf(m_blk, __uint_as_float(raw[e]));
-          } else {
+      for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + (uint32_t)(c * 32), raw[c]);
+      tmem_ld_wait();
+      // P = exp2(S * scale - m) as bf16 / fp16 pairs over the first 64 columns of S; packed fp32 arithmetic, one
+      // special-function instruction per exponential, one conversion per pair.  Two instantiations: with the mask test
+      // inside one, every element pays a compare and a select.
+      float l0, l1;
+      uint32_t pk[4][16];
+      auto chunk_p = [&](auto masked, int c, float neg_m) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (c * 32 + e < lim) m_blk = fmaxf(m_blk, __uint_as_float(raw[e]));
+        for (int e = 0; e < 32; e += 2) {
+          float x0, x1;
+          fma2(x0, x1, __uint_as_float(raw[c][e]), __uint_as_float(raw[c][e + 1]), p.scale_log2, neg_m);
+          float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
+          if constexpr (decltype(masked)::value) {
+            if (c * 32 + e >= lim) p0 = 0.f;
+            if (c * 32 + e + 1 >= lim) p1 = 0.f;
           }
-        };
-        tmem_ld32(s_addr, ra);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 32u, rb);
-        chunk_max(ra, 0);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 64u, ra);
-        chunk_max(rb, 1);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 96u, rb);
-        chunk_max(ra, 2);
-        tmem_ld_wait();
-        chunk_max(rb, 3);
-      }
-      const float m_new = fmaxf(m_ref, m_blk * p.scale_log2);
-      // P of the previous block must have been consumed (and O updated) before P is rewritten or O rescaled
-      if (j > 0 && !wait_all(&pv_done[t], (uint32_t)((j - 1) & 1))) { ok = false; break; }
-      const bool raise = m_new - m_ref > kRescaleThreshold;      // also true for the first finite maximum
-      if (__any_sync(0xffffffffu, raise)) {
-        const float alpha = raise ? exp2f(m_ref - m_new) : 1.f;   // 0 when m_ref = -inf
-        if (j > 0) {
-          tc_fence_after();
-#pragma unroll
-          for (int c = 0; c < AD / 32; ++c) {
-            uint32_t raw[32];
-            tmem_ld32(o_addr + (uint32_t)(c * 32), raw);
-            tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) raw[e] = __float_as_uint(__uint_as_float(raw[e]) * alpha);
-            tmem_st32(o_addr + (uint32_t)(c * 32), raw);
-          }
-          tmem_st_wait();
+          add2(l0, l1, p0, p1);
+          pk[c][e >> 1] = pack2<T>(p0, p1);
         }
-        if (raise) {
-          l_run *= alpha;
-          m_ref = m_new;
-        }
-      }
-      const float m_use = m_ref == -INFINITY ? 0.f : m_ref;       // row without any visible key so far
-      // pass 2: P = exp2(S * scale - m) as bf16/fp16 into the swizzled K-major tile; packed fp32 arithmetic, one
-      // special-function instruction per exponential, one conversion per pair
-      float l0 = 0.f, l1 = 0.f;
-      {
-        uint32_t ra[32], rb[32];
-        const float neg_m = -m_use;
-        auto chunk_p = [&](const uint32_t (&raw)[32], int c) {
-          uint32_t pk[16];
+      };
+      auto block = [&](auto masked) {
+        // The first part is computed against the reference maximum as it stands, while the block's own maximum is found
+        // beside it (four chains of three-input maxima under the special-function unit's shadow): m is raised in the first
+        // block and hardly ever after it, and only then is the first part computed again.
+        l0 = l1 = 0.f;
+        const float m_old = m_ref == -INFINITY ? 0.f : m_ref;
+#pragma unroll
+        for (int c = 0; c < kFirstPart / 32; ++c) chunk_p(masked, c, -m_old);
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int e = 0; e < 32; e += 2) {
-            float x0, x1;
-            fma2(x0, x1, __uint_as_float(raw[e]), __uint_as_float(raw[e + 1]), p.scale_log2, neg_m);
-            float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
-            if (!full) {
-              if (c * 32 + e >= lim) p0 = 0.f;
-              if (c * 32 + e + 1 >= lim) p1 = 0.f;
+            float a = __uint_as_float(raw[c][e]), b2 = __uint_as_float(raw[c][e + 1]);
+            if constexpr (decltype(masked)::value) {
+              if (c * 32 + e >= lim) a = -INFINITY;
+              if (c * 32 + e + 1 >= lim) b2 = -INFINITY;
             }
-            add2(l0, l1, p0, p1);
-            pk[e >> 1] = pack2<T>(p0, p1);
+            mx[(e >> 1) & 3] = max3(mx[(e >> 1) & 3], a, b2);
           }
+        const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        const float m_new = fmaxf(m_ref, m_blk * p.scale_log2);
+        const bool raise = m_new - m_ref > kRescaleThreshold;      // also true for the first finite maximum
+        if (__any_sync(0xffffffffu, raise)) {
+          const float alpha = raise ? exp2f(m_ref - m_new) : 1.f;   // 0 when m_ref = -inf
+          if (j > 0) {
 #pragma unroll
-          for (int g8 = 0; g8 < 4; ++g8) {
-            const int c8 = c * 4 + g8;
-            const int atom = c8 >> 3, ch = c8 & 7;
-            *reinterpret_cast<uint4*>(prow + (size_t)atom * (kTile / 2) + (size_t)((ch ^ (r & 7)) * 16)) =
-                make_uint4(pk[g8 * 4], pk[g8 * 4 + 1], pk[g8 * 4 + 2], pk[g8 * 4 + 3]);
+            for (int c = 0; c < AD / 16; ++c) {
+              uint32_t o16[16];
+              tmem_ld16(o_addr + (uint32_t)(c * 16), o16);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o16[e] = __float_as_uint(__uint_as_float(o16[e]) * alpha);
+              tmem_st16(o_addr + (uint32_t)(c * 16), o16);
+            }
           }
-        };
-        tmem_ld32(s_addr, ra);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 32u, rb);
-        chunk_p(ra, 0);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 64u, ra);
-        chunk_p(rb, 1);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 96u, rb);
-        chunk_p(ra, 2);
-        tmem_ld_wait();
-        chunk_p(rb, 3);
-      }
-      const float l_blk = l0 + l1;
-      l_run += l_blk;
+          if (raise) {
+            l_run *= alpha;
+            m_ref = m_new;
+          }
+          l0 = l1 = 0.f;
+          const float m_use = m_ref == -INFINITY ? 0.f : m_ref;     // row without any visible key so far
+#pragma unroll
+          for (int c = 0; c < kFirstPart / 32; ++c) chunk_p(masked, c, -m_use);
+        }
+#pragma unroll
+        for (int c = 0; c < kFirstPart / 32; ++c) tmem_st16(s_addr + (uint32_t)(c * 16), pk[c]);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[2 * t]);
+        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+#pragma unroll
+        for (int c = kFirstPart / 32; c < 4; ++c) {
+          chunk_p(masked, c, -m_use);
+          tmem_st16(s_addr + (uint32_t)(c * 16), pk[c]);
+        }
+      };
+      if (full) block(std::false_type{});
+      else block(std::true_type{});
+      l_run += l0 + l1;
+      tmem_st_wait();
       tc_fence_before();
-      // make the generic-proxy writes of P visible to the tensor core (async proxy), then signal
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&s_free[t]);          // the tensor core may overwrite this S buffer
-        mbar_arrive(&p_ready[t]);
-      }
+      if (lane == 0) mbar_arrive(&p_ready[2 * t + 1]);
     }
-    if (ok && n_blocks > 0) ok = wait_all(&pv_done[t], (uint32_t)((n_blocks - 1) & 1));
+    if (ok && n_blocks > 0) ok = wait_all(&mma_done[t], (uint32_t)(n_blocks & 1));
     if (ok && n_blocks > 0) {
       tc_fence_after();
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
@@ -369,6 +371,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     tmem_dealloc(tmem_base, kAttnTmemCols);
   }
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
+}
+
+template <typename K>
+int fwd_setup(K kern) {
+  cudaFuncAttributes at;
+  cudaError_t e = cudaFuncGetAttributes(&at, kern);
+  if (e != cudaSuccess) return (int)e;
+  if (at.numRegs < kLaunchRegs) return (int)cudaErrorNotSupported;   // the register split would wait for ever
+  return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
 }
 
 }  // namespace
@@ -421,23 +432,13 @@ extern "C" int b200_flash_attn_fwd(const b200_attn_t* a, void* out, float* lse, 
   const long long grid = (long long)a->B * a->H * p.q_pairs;
   if (grid > 2147483647ll) return (int)cudaErrorNotSupported;
   if (bf16) {
-    static bool set = false;
-    auto kern = attn_fwd_kernel<__nv_bfloat16>;
-    if (!set) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
-      if (e != cudaSuccess) return (int)e;
-      set = true;
-    }
-    kern<<<(unsigned)grid, kAttnThreads, kAttnSmem, stream>>>(mq, mk, mv, (__nv_bfloat16*)out, p);
+    static const int e = fwd_setup(attn_fwd_kernel<__nv_bfloat16>);
+    if (e != 0) return e;
+    attn_fwd_kernel<__nv_bfloat16><<<(unsigned)grid, kAttnThreads, kAttnSmem, stream>>>(mq, mk, mv, (__nv_bfloat16*)out, p);
   } else {
-    static bool set = false;
-    auto kern = attn_fwd_kernel<__half>;
-    if (!set) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
-      if (e != cudaSuccess) return (int)e;
-      set = true;
-    }
-    kern<<<(unsigned)grid, kAttnThreads, kAttnSmem, stream>>>(mq, mk, mv, (__half*)out, p);
+    static const int e = fwd_setup(attn_fwd_kernel<__half>);
+    if (e != 0) return e;
+    attn_fwd_kernel<__half><<<(unsigned)grid, kAttnThreads, kAttnSmem, stream>>>(mq, mk, mv, (__half*)out, p);
   }
   B200K_LAUNCH_RET();
 }
