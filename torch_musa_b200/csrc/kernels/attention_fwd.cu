@@ -162,7 +162,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const uint64_t q_desc = make_desc(smem_u32(sQ), 16, 1024);             // K-major tiles; + (bytes >> 4) for an offset
       const uint64_t k_desc = make_desc(smem_u32(sR), 16, 1024);
       const uint64_t v_desc = make_desc(smem_u32(sR), kTile / 2, 1024);      // MN-major
-      auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
+      auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity, abort_flag); };
       auto ring_wait = [&](int n) { return wait(&r_full[n % kRing], (uint32_t)((n / kRing) & 1)); };
       auto issue_s = [&](int t, int n) {     // S_t = Q_t K^T with K in ring item n
         const uint64_t qa = q_desc + (uint32_t)(t * (kTile >> 4)), ka = k_desc + (uint32_t)((n % kRing) * (kTile >> 4));

@@ -183,26 +183,27 @@ conv_pix_kernel(const __grid_constant__ Maps maps, const __grid_constant__ PixPa
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        if (!mbar_wait(&s.tempty[acc], acc_phase ^ 1, s.abort_flag)) { ok = false; break; }
+    const bool issuer = elect_one();
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      if (!mbar_wait_warp(&s.tempty[acc], acc_phase ^ 1, s.abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
+      for (int ks = 0; ks < k_steps; ++ks) {
+        if (!mbar_wait_warp(&s.full[stage], phase, s.abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
-        for (int ks = 0; ks < k_steps; ++ks) {
-          if (!mbar_wait(&s.full[stage], phase, s.abort_flag)) { ok = false; break; }
-          tc_fence_after();
+        if (issuer) {
           issue_stage<true, B_KMAJOR>(tmem_d, smem_u32(s.a + stage * kATile), smem_u32(s.b + stage * kBTile), p.idesc,
-                                      ks == 0);
+                                    ks == 0);
           umma_commit(&s.empty[stage]);
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
-        umma_commit(&s.tfull[acc]);
-        if (++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (issuer) umma_commit(&s.tfull[acc]);
+      if (++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
     }
     __syncwarp();
   } else {
@@ -321,28 +322,29 @@ conv_wgrad_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Wgr
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        int mt, tap_i, nc, s0, s1;
-        decode(tile, mt, tap_i, nc, s0, s1);
-        if (!mbar_wait(&s.tempty[acc], acc_phase ^ 1, s.abort_flag)) { ok = false; break; }
+    const bool issuer = elect_one();
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      int mt, tap_i, nc, s0, s1;
+      decode(tile, mt, tap_i, nc, s0, s1);
+      if (!mbar_wait_warp(&s.tempty[acc], acc_phase ^ 1, s.abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
+      for (int st = s0; st < s1; ++st) {
+        if (!mbar_wait_warp(&s.full[stage], phase, s.abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
-        for (int st = s0; st < s1; ++st) {
-          if (!mbar_wait(&s.full[stage], phase, s.abort_flag)) { ok = false; break; }
-          tc_fence_after();
+        if (issuer) {
           issue_stage<false, false>(tmem_d, smem_u32(s.a + stage * kATile), smem_u32(s.b + stage * kBTile), p.idesc,
-                                    st == s0);
+                                  st == s0);
           umma_commit(&s.empty[stage]);
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
-        umma_commit(&s.tfull[acc]);
-        if (++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (issuer) umma_commit(&s.tfull[acc]);
+      if (++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
     }
     __syncwarp();
   } else {
@@ -366,10 +368,13 @@ conv_wgrad_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Wgr
         tmem_ld32(taddr + (uint32_t)(c * 32), raw);
         tmem_ld_wait();
         if (k < p.c_out && s1 > s0) {
-          const int nvalid = min(32, p.c_in - col0);
+          const int nvalid = min(32, p.c_in - col0);   // a multiple of 8
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (e < nvalid) atomicAdd(drow + c * 32 + e, __uint_as_float(raw[e]));
+          for (int e = 0; e < 32; e += 4)
+            if (e < nvalid)
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(drow + c * 32 + e), "f"(__uint_as_float(raw[e])),
+                           "f"(__uint_as_float(raw[e + 1])), "f"(__uint_as_float(raw[e + 2])), "f"(__uint_as_float(raw[e + 3]))
+                           : "memory");
         }
       }
       tc_fence_before();

@@ -103,7 +103,10 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint6
 // One lane of the (converged) warp.  The roles that issue MMAs or TMA copies run their loops with the whole warp and guard
 // only the asynchronous instructions with this predicate: inside an `if (lane == 0)` block the addresses and descriptors are
 // per-thread values, and moving them to the uniform registers that these instructions take costs more than the 64 clocks that
-// an M128 N128 K16 product runs for.
+// an M128 N128 K16 product runs for (measured: 75 clocks from one product to the next, 65 with the elected lane).  Before ->
+// after with nothing else changed: fp8 linear layer 4096 x 14336 x 4096 550 -> 494 us, grouped expert GEMMs in training
+// 9.00 -> 8.51 ms, 3x3 convolution with batch norm in training (with vector reductions in its weight gradient) 418 -> 405 us;
+// 0.7 to 1.2 % on the M256 N256 pair kernel, whose products are long enough to hide most of it.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(
@@ -112,6 +115,10 @@ __device__ __forceinline__ bool elect_one() {
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(p));
   return p != 0;
+}
+// mbar_wait by a converged warp: every lane gets the same answer
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 // Arrives on the mbarrier once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {

@@ -104,24 +104,25 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        const int slot = kb & 1;
-        // the promotion warps must have drained this accumulator (block kb - 2)
-        if (!mbar_wait(&tempty_bar[slot], (uint32_t)(((kb >> 1) & 1) ^ 1), abort_flag)) break;
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) break;
-        tc_fence_after();
-        const uint32_t sa = smem_u32(smem_a + stage * kF8Tile), sb = smem_u32(smem_b + stage * kF8Tile);
-        const uint32_t tmem_d = tmem_base + (uint32_t)(slot * FN);
+    const bool issuer = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int kb = 0; kb < k_blocks; ++kb) {
+      const int slot = kb & 1;
+      // the promotion warps must have drained this accumulator (block kb - 2)
+      if (!mbar_wait_warp(&tempty_bar[slot], (uint32_t)(((kb >> 1) & 1) ^ 1), abort_flag)) break;
+      if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) break;
+      tc_fence_after();
+      const uint32_t sa = smem_u32(smem_a + stage * kF8Tile), sb = smem_u32(smem_b + stage * kF8Tile);
+      const uint32_t tmem_d = tmem_base + (uint32_t)(slot * FN);
+      if (issuer) {
 #pragma unroll
         for (int kk = 0; kk < FK / 32; ++kk)
           umma_f8(tmem_d, make_desc(sa + kk * 32, 16, 1024), make_desc(sb + kk * 32, 16, 1024), p.idesc, kk != 0 ? 1u : 0u);
         umma_commit(&empty_bar[stage]);
         umma_commit(&tfull_bar[slot]);
-        if (++stage == kF8Stages) { stage = 0; phase ^= 1; }
       }
+      if (++stage == kF8Stages) { stage = 0; phase ^= 1; }
     }
     __syncwarp();
   } else {

@@ -166,20 +166,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (whole warp waits; lane 0 issues)
+    // ------------------------------------------------------------ MMA issuer (the whole warp waits, one lane issues)
     constexpr bool A_KMAJOR = !RAGGED_K;
     constexpr bool BK_MAJOR = !RAGGED_K && B_KMAJOR;
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
     bool ok = true;
-    // lane 0 waits, the warp takes its answer: the lanes can never disagree about leaving the loop
-    auto warp_wait = [&](uint64_t* bar, uint32_t parity) {
-      int w = 1;
-      if (lane == 0) w = mbar_wait(bar, parity, abort_flag) ? 1 : 0;
-      w = __shfl_sync(0xffffffffu, w, 0);
-      __syncwarp();
-      return w != 0;
-    };
+    const bool issuer = elect_one();
+    auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity, abort_flag); };
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       int g, m0, n0, krow0, kbs, kcount;
       locate(tile, g, m0, n0, krow0, kbs, kcount);
@@ -205,7 +199,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
           __syncwarp();
         }
-        if (lane == 0) {
+        if (issuer) {
           const uint32_t sa = smem_u32(pa);
           const uint32_t sb = smem_u32(pb);
 #pragma unroll
@@ -220,7 +214,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
       if (!ok) break;
-      if (lane == 0) umma_commit(&tfull_bar[acc]);
+      if (issuer) umma_commit(&tfull_bar[acc]);
       __syncwarp();
       if (++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
     }

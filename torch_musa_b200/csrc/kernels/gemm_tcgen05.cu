@@ -131,21 +131,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        const int kb0 = (tile / tiles_all_batches) * p.kb_per_split;
-        const int kb1 = min(k_blocks, kb0 + p.kb_per_split);
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+    const bool issuer = elect_one();
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      const int kb0 = (tile / tiles_all_batches) * p.kb_per_split;
+      const int kb1 = min(k_blocks, kb0 + p.kb_per_split);
+      if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem_a + stage * kATileBytes);
-          const uint32_t sb = smem_u32(smem_b + stage * kBTileBytes);
+        const uint32_t sa = smem_u32(smem_a + stage * kATileBytes);
+        const uint32_t sb = smem_u32(smem_b + stage * kBTileBytes);
+        if (issuer) {
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
             // K-major: 16 elements = 32 B inside the 128-byte swizzle row; SBO = 8 rows x 128 B.
@@ -156,12 +157,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             else umma_f16(tmem_d, adesc, bdesc, p.idesc, (kb > kb0 || kk != 0) ? 1u : 0u);
           }
           umma_commit(&empty_bar[stage]);  // slot reusable once these MMAs have read it
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
-        umma_commit(&tfull_bar[acc]);  // accumulator complete
-        if (++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (issuer) umma_commit(&tfull_bar[acc]);  // accumulator complete
+      if (++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
     }
     __syncwarp();
   } else {

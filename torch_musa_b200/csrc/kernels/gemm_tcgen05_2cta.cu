@@ -491,7 +491,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    if (leader) {
+      const bool issuer = elect_one();
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
@@ -500,27 +501,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       while (more && ok) {
         const int kb0 = (tile / tiles_all_batches) * p.kb_per_split;
         const int kb1 = min(k_blocks, kb0 + p.kb_per_split);
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem_a + stage * C::kATile);
           const uint32_t sb = smem_u32(smem_b + stage * C::kBTile);
+          if (issuer) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t adesc = A_KMAJOR ? make_desc(sa + kk * 32, 16, 1024) : make_desc(sa + kk * 2048, 8192, 1024);
-            const uint64_t bdesc = B_KMAJOR ? make_desc(sb + kk * 32, 16, 1024) : make_desc(sb + kk * 2048, 8192, 1024);
-            umma_f16_pair(tmem_d, adesc, bdesc, p.idesc, (kb > kb0 || kk != 0) ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk) {
+              const uint64_t adesc = A_KMAJOR ? make_desc(sa + kk * 32, 16, 1024) : make_desc(sa + kk * 2048, 8192, 1024);
+              const uint64_t bdesc = B_KMAJOR ? make_desc(sb + kk * 32, 16, 1024) : make_desc(sb + kk * 2048, 8192, 1024);
+              umma_f16_pair(tmem_d, adesc, bdesc, p.idesc, (kb > kb0 || kk != 0) ? 1u : 0u);
+            }
+            umma_commit_pair(&empty_bar[stage], 3);  // frees this slot in both CTAs
           }
-          umma_commit_pair(&empty_bar[stage], 3);  // frees this slot in both CTAs
           if (++stage == C::kStages) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit_pair(&tfull_bar[acc], 3);  // accumulator complete in both CTAs
+        if (issuer) umma_commit_pair(&tfull_bar[acc], 3);  // accumulator complete in both CTAs
         if (++acc == C::kAcc) { acc = 0; acc_phase ^= 1; }
-        more = next_tile(cur, dynamic, tile, n_pairs, total_tiles, abort_flag);
+        // lane 0 reads the scheduler's answer for the whole warp
+        int next = tile, go = 0;
+        if (lane == 0) go = next_tile(cur, dynamic, next, n_pairs, total_tiles, abort_flag) ? 1 : 0;
+        tile = __shfl_sync(0xffffffffu, next, 0);
+        more = __shfl_sync(0xffffffffu, go, 0) != 0;
       }
     }
     __syncwarp();
@@ -747,7 +754,7 @@ int gemm_forced_config_exchange(int c) { return g_forced_config.exchange(c); }
 // Chooses the kernel family and the split-K factor.
 // Family: waves x per-wave cost; per wave the pair kernel is ~15% cheaper (measured 1.42-1.54 against 1.22-1.43
 // PFLOP/s on 4096-row bf16 problems) because each SM reads half of B.  256x128 pair tiles were measured too and
-// rejected: an N=128 instruction is no faster per column than N=256, so they ran at 0.7-0.98 PFLOP/s.
+// rejected (0.7-0.98 PFLOP/s, while the products were still issued from an `if (lane == 0)` block: see elect_one).
 // Split-K: when the output has fewer tiles than half the machine and K is long (weight gradients of
 // convolutions and of small linear layers: K = batch x pixels), K is cut so that every SM (pair) gets a slice.
 GemmPlan gemm_plan(const b200_gemm_desc_t* g) {
