@@ -222,3 +222,28 @@ def test_forward_maximum_rises_with_every_block(bw, dev, native_sdp, S, causal, 
     assert (out.float().cpu() - ref).abs().max() < tol
     bw.synchronize()
     assert bw._C._gemm_status(False) == 0
+
+
+@pytest.mark.parametrize("Sq,Sk,H,Hkv", [(1, 1, 1, 1), (129, 129, 4, 1), (257, 385, 2, 2), (64, 257, 4, 2), (513, 127, 2, 1)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_backward_edges(bw, dev, native_sdp, Sq, Sk, H, Hkv, causal):
+    """Remainders of the query and key blocks, one and several pairs per block of keys, grouped heads; causal with fewer
+    and with more keys than queries (keys without any query get zero gradients)."""
+    torch.manual_seed(6)
+    q, g = (torch.randn(2, Sq, H, 128).bfloat16().transpose(1, 2) for _ in range(2))
+    k, v = (torch.randn(2, Sk, Hkv, 128).bfloat16().transpose(1, 2) for _ in range(2))
+    qr, kr, vr = (t.float().requires_grad_() for t in (q, k, v))
+    ref, _ = ref_attention(qr, kr, vr, causal)
+    ref.backward(g.float())
+    qd, kd, vd = (t.to(dev).requires_grad_() for t in (q, k, v))
+    before = bw._C._native_sdp_backward_calls()
+    out = F.scaled_dot_product_attention(qd, kd, vd, is_causal=causal, enable_gqa=(H != Hkv))
+    out.backward(g.to(dev))
+    assert bw._C._native_sdp_backward_calls() == before + 1
+    for name, a, b in (("dq", qd.grad, qr.grad), ("dk", kd.grad, kr.grad), ("dv", vd.grad, vr.grad)):
+        # P and dS are rounded to bf16 (2^-9) before they are multiplied, the result is rounded again: 3e-2 of the largest entry
+        # as above; an exact zero everywhere (one query and one key: the softmax is constant) may come out as rounding noise
+        err = (a.float().cpu() - b).abs().max()
+        assert err < 3e-2 * max(float(b.abs().max()), 1.0), (name, float(err))
+    bw.synchronize()
+    assert bw._C._gemm_status(False) == 0

@@ -6,20 +6,32 @@
 // computed transposed, keys along the 128 TMEM lanes, so that one thread owns one key row:
 //   S^T  = K Q^T          tcgen05.mma, both operands K-major                         -> TMEM columns [0, 128)
 //   dP^T = V dO^T         the same shape                                             -> TMEM columns [128, 256)
-//   P^T  = exp2(S^T * scale - lse[q]),  dS^T = P^T * (dP^T - delta[q]) * scale       two warpgroups, half of the
-//                         query columns each; both written as bf16 into shared memory in the layout of an A operand
-//   dV  += P^T dO         A = P^T (K-major over queries), B = dO read MN-major       -> TMEM columns [256, 384)
-//   dK  += dS^T Q         A = dS^T, B = Q read MN-major                              -> TMEM columns [384, 512)
+//   P^T  = exp2(S^T * scale - lse[q])     two warpgroups, half of the query columns each; 16-bit pairs into TMEM over S^T
+//   dV  += P^T dO         A = P^T from TMEM, B = dO read MN-major                    -> TMEM columns [256, 384)
+//   dS^T = P^T * (dP^T - delta[q]) * scale   the same warpgroups; 16-bit into shared memory in the layout of an A operand
 //   dQ   = dS K           A = dS^T read MN-major, B = K read MN-major, fresh         -> TMEM columns [128, 256) again
-// dQ of this (query block, key block) pair is staged as fp32 in the shared memory that P^T / dS^T occupied and added
-// to an fp32 buffer in global memory by TMA reductions (cp.reduce.async.bulk.tensor ... add); the caller zeroes that
-// buffer and converts it afterwards.  delta = rowsum(dO * O) comes
-// from a small preprocessing kernel.  Q and dO stream through a three-slot TMA ring; every wait is bounded.
+//   dK  += dS^T Q         A = dS^T, B = Q read MN-major                              -> TMEM columns [384, 512)
+// A third warpgroup takes dQ of every (query block, key block) pair out of TMEM, stages it as fp32 in two 16 KB boxes of
+// its own and adds it to an fp32 buffer in global memory by TMA reductions (cp.reduce.async.bulk.tensor ... add); the
+// caller converts that buffer afterwards.  delta = rowsum(dO * O) comes from a small kernel that also zeroes the buffer.
+//
+// What runs beside what, per pair: S^T of the next pair is issued right after dV, so its exponentials run while the tensor
+// core does dQ and dK; dQ leaves TMEM into registers while dK runs, which frees its columns for the next dP^T; the staging
+// and the reductions have the whole next pair's time.  The loop that remains is dS -> dQ -> (dQ out of TMEM, under dK) ->
+// next dP^T -> next dS.  P^T in TMEM instead of shared memory pays for the separate staging boxes.  Q streams through two
+// slots, dO through one (it is free after dV), lse and delta through a two-slot ring filled by a warp of its own; every wait
+// is bounded.
+// What bounds it now is shared memory: per pair the products read 288 KB, the tiles of Q and dO bring 64, dS^T 32 and the
+// staged dQ 128, which at 128 bytes per clock is 4000 clocks beside 2560 of products (4400 measured, at 32 heads x 4096 x
+// 128).  bf16, before -> after: causal 672 -> 351 us (980 TFLOP/s), full 1310 -> 640.  Registers: 96 for the warps that
+// issue keep their descriptors out of local memory, whose traffic goes through the same shared-memory path (with 56: +9 %).
+// Tried and not kept: starting each block of keys at another query block (+10 %).
 //
 // Parity: the reference calls a closed vendor flash backward (reference torch_musa/csrc/aten/ops/attention/mudnn/SDP.cpp:678-845).
 #include "attention_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace b200k {
 namespace {
@@ -28,11 +40,14 @@ using namespace attndev;
 
 constexpr int BQ = 128, BK = 128, BD = 128;
 constexpr int kTile = 128 * 128 * 2;
-constexpr int kRing = 3;
-constexpr int kBwdSmem = 2 * kTile /*K, V*/ + kRing * kTile /*Q, dO ring*/ + 2 * kTile /*P^T, dS^T*/ + 1024 +
-                         2 * 128 * 4 /*lse, delta*/ + 128;
+constexpr int kStage = 128 * 32 * 4;                  // 16 KB: 32 fp32 columns of dQ
+constexpr int kBwdSlack = 768;                        // for the alignment of the tiles to 1024 bytes (checked by the kernel)
+constexpr int kBwdSmem = 2 * kTile /*K, V*/ + 2 * kTile /*Q*/ + kTile /*dO*/ + kTile /*dS^T*/ + 2 * kStage /*dQ*/ +
+                         2 * 2 * 128 * 4 /*lse, delta*/ + 256 /*barriers*/ + kBwdSlack;
 static_assert(kBwdSmem <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
-constexpr int kBwdThreads = 320;
+constexpr int kBwdThreads = 512;                      // 2 compute warpgroups, dQ warpgroup, TMA / MMA / lse-delta warps
+constexpr int kComputeRegs = 136, kDqRegs = 144, kOtherRegs = 96;    // register split (sum: what 128 per thread brings)
+constexpr int kLaunchRegs = (2 * kComputeRegs + kDqRegs + kOtherRegs + 3) / 4;
 constexpr uint32_t kBwdTmemCols = 512;
 
 struct BwdParams {
@@ -41,7 +56,7 @@ struct BwdParams {
   float scale, scale_log2;
   const float* lse;       // [B, H, Sq] natural log
   const float* delta;     // [B, H, Sq]
-  float* dq;              // [B, H, Sq, 128] fp32, zeroed
+  float* dq;              // [B, H, Sq, 128] fp32
   int64_t dk_sb, dk_sh, dk_ss, dv_sb, dv_sh, dv_ss;
   int kv_blocks, q_blocks;
   int* status;
@@ -66,26 +81,34 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 const __grid_constant__ CUtensorMap tmap_dq, T* __restrict__ dk, T* __restrict__ dv, const BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  if (smem - smem_raw > kBwdSlack) {        // cannot happen while the kernel has no static shared memory
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1);
+    return;
+  }
   uint8_t* sK = smem;
   uint8_t* sV = smem + kTile;
-  uint8_t* sR = smem + 2 * kTile;                    // [kRing][kTile]: Q_i, dO_i, Q_{i+1}, ...
-  uint8_t* sP = smem + (2 + kRing) * kTile;          // P^T  [keys x queries]
-  uint8_t* sS = smem + (3 + kRing) * kTile;          // dS^T [keys x queries]
-  float* s_lse = reinterpret_cast<float*>(smem + (4 + kRing) * kTile);   // [128]
-  float* s_dlt = s_lse + 128;                                              // [128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_dlt + 128);
+  uint8_t* sQ = smem + 2 * kTile;                    // [2][kTile]
+  uint8_t* sdO = smem + 4 * kTile;
+  uint8_t* sS = smem + 5 * kTile;                    // dS^T [keys x queries]
+  uint8_t* sStage = smem + 6 * kTile;                // [2][kStage] fp32 dQ
+  float* s_lse = reinterpret_cast<float*>(smem + 6 * kTile + 2 * kStage);   // [2][128]
+  float* s_dlt = s_lse + 2 * 128;                                             // [2][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_dlt + 2 * 128);
   uint64_t* kv_full = bars;                  // 1
-  uint64_t* r_full = bars + 1;               // [kRing]
-  uint64_t* r_empty = r_full + kRing;        // [kRing]  tcgen05.commit
-  uint64_t* s_full = r_empty + kRing;        // tcgen05.commit: S^T ready
-  uint64_t* dp_full = s_full + 1;            // tcgen05.commit: dP^T ready
-  uint64_t* s_free = dp_full + 1;            // 8 warps: S^T read
-  uint64_t* p_ready = s_free + 1;            // 8 warps: P^T in shared memory
-  uint64_t* ds_ready = p_ready + 1;          // 8 warps: dS^T in shared memory, dP^T read
-  uint64_t* mma2_done = ds_ready + 1;        // tcgen05.commit: dV, dK, dQ of this pair complete
-  uint64_t* dq_drained = mma2_done + 1;      // 8 warps: dQ read out of TMEM
-  uint64_t* stage_free = dq_drained + 1;     // one thread: the TMA reduction has read the staged dQ
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stage_free + 1);
+  uint64_t* q_full = bars + 1;               // [2]
+  uint64_t* q_empty = bars + 3;              // [2]  tcgen05.commit after dK
+  uint64_t* do_full = bars + 5;              // 1
+  uint64_t* do_empty = bars + 6;             // tcgen05.commit after dV
+  uint64_t* s_full = bars + 7;               // tcgen05.commit: S^T
+  uint64_t* dp_full = bars + 8;              // tcgen05.commit: dP^T (and with it everything issued before)
+  uint64_t* p_ready = bars + 9;              // 8 warps: P^T in TMEM
+  uint64_t* ds_ready = bars + 10;            // 8 warps: dS^T in shared memory, dP^T read
+  uint64_t* dq_full = bars + 11;             // tcgen05.commit: dQ
+  uint64_t* dq_drained = bars + 12;          // 4 warps: dQ is in registers
+  uint64_t* all_done = bars + 13;            // tcgen05.commit: dV, dK complete
+  uint64_t* ld_full = bars + 14;             // [2]  lse and delta of a query block are there
+  uint64_t* ld_empty = bars + 16;            // [2]  8 warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -114,18 +137,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     mbar_init(kv_full, 1);
-    for (int s = 0; s < kRing; ++s) {
-      mbar_init(&r_full[s], 1);
-      mbar_init(&r_empty[s], 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+      mbar_init(&ld_full[i], 1);
+      mbar_init(&ld_empty[i], 8);
     }
+    mbar_init(do_full, 1);
+    mbar_init(do_empty, 1);
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
-    mbar_init(s_free, 8);
     mbar_init(p_ready, 8);
     mbar_init(ds_ready, 8);
-    mbar_init(mma2_done, 1);
-    mbar_init(dq_drained, 8);
-    mbar_init(stage_free, 1);
+    mbar_init(dq_full, 1);
+    mbar_init(dq_drained, 4);
+    mbar_init(all_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     prefetch_tmap(&tmap_q);
     prefetch_tmap(&tmap_k);
@@ -133,7 +159,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     prefetch_tmap(&tmap_do);
     prefetch_tmap(&tmap_dq);
   }
-  if (warp == 9) {
+  if (warp == 13) {
     tmem_alloc(tmem_slot, kBwdTmemCols);
     tmem_relinquish();
   }
@@ -143,146 +169,201 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
   constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 384;
 
-  if (warp == 8) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0 && n_it > 0) {
-      mbar_expect_tx(kv_full, 2 * kTile);
-      tma_load_4d(sK, &tmap_k, kv_full, 0, koff + k0, hk, bt);
-      tma_load_4d(sK + kTile / 2, &tmap_k, kv_full, 64, koff + k0, hk, bt);
-      tma_load_4d(sV, &tmap_v, kv_full, 0, koff + k0, hk, bt);
-      tma_load_4d(sV + kTile / 2, &tmap_v, kv_full, 64, koff + k0, hk, bt);
-      for (int n = 0; n < 2 * n_it; ++n) {
-        const int st = n % kRing;
-        if (!mbar_wait(&r_empty[st], (uint32_t)(((n / kRing) & 1) ^ 1), abort_flag)) break;
-        mbar_expect_tx(&r_full[st], kTile);
-        const int it = n >> 1;
-        const int h = hk * G + it / n_i;
-        const int q0 = (i0 + it % n_i) * BQ;
-        const CUtensorMap* map = (n & 1) ? &tmap_do : &tmap_q;
-        tma_load_4d(sR + st * kTile, map, &r_full[st], 0, qoff + q0, h, bt);
-        tma_load_4d(sR + st * kTile + kTile / 2, map, &r_full[st], 64, qoff + q0, h, bt);
+  if (warp >= 12) {
+    regs_dec<kOtherRegs>();
+    if (warp == 12) {
+      // ------------------------------------------------------------ TMA producer
+      if (lane == 0 && n_it > 0) {
+        mbar_expect_tx(kv_full, 2 * kTile);
+        tma_load_4d(sK, &tmap_k, kv_full, 0, koff + k0, hk, bt);
+        tma_load_4d(sK + kTile / 2, &tmap_k, kv_full, 64, koff + k0, hk, bt);
+        tma_load_4d(sV, &tmap_v, kv_full, 0, koff + k0, hk, bt);
+        tma_load_4d(sV + kTile / 2, &tmap_v, kv_full, 64, koff + k0, hk, bt);
+        int h = hk * G, i = 0;
+        for (int it = 0; it < n_it; ++it) {
+          const int q0 = (i0 + i) * BQ, st = it & 1;
+          if (!mbar_wait(&q_empty[st], (uint32_t)(((it >> 1) & 1) ^ 1), abort_flag)) break;
+          mbar_expect_tx(&q_full[st], kTile);
+          tma_load_4d(sQ + st * kTile, &tmap_q, &q_full[st], 0, qoff + q0, h, bt);
+          tma_load_4d(sQ + st * kTile + kTile / 2, &tmap_q, &q_full[st], 64, qoff + q0, h, bt);
+          if (!mbar_wait(do_empty, (uint32_t)((it & 1) ^ 1), abort_flag)) break;
+          mbar_expect_tx(do_full, kTile);
+          tma_load_4d(sdO, &tmap_do, do_full, 0, qoff + q0, h, bt);
+          tma_load_4d(sdO + kTile / 2, &tmap_do, do_full, 64, qoff + q0, h, bt);
+          if (++i == n_i) { i = 0; ++h; }
+        }
       }
-    }
-    __syncwarp();
-  } else if (warp == 9) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_it > 0) {
-      const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      const uint32_t idesc_kk = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-      const uint32_t idesc_kmn = idesc_kk | (1u << 16);                 // B read MN-major
-      const uint32_t idesc_mnmn = idesc_kk | (1u << 15) | (1u << 16);   // A and B read MN-major
-      auto ring_wait = [&](int n) { return mbar_wait(&r_full[n % kRing], (uint32_t)((n / kRing) & 1), abort_flag); };
-      // D = A B^T with both tiles K-major (two 64-column atoms, 32 bytes per k16 step)
-      auto mma_kk = [&](uint32_t dcol, const uint8_t* a, const uint8_t* bt) {
-        const uint32_t aa = smem_u32(a), ba = smem_u32(bt);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t off = (uint32_t)(kk >> 2) * (kTile / 2) + (uint32_t)(kk & 3) * 32;
-          umma_f16(tmem_base + dcol, make_desc(aa + off, 16, 1024), make_desc(ba + off, 16, 1024), idesc_kk, kk != 0 ? 1u : 0u);
-        }
-      };
-      // D (+)= A B with A K-major and B a [k rows x n columns] tile read MN-major (16 k rows = 2048 bytes per step)
-      auto mma_kmn = [&](uint32_t dcol, const uint8_t* a, const uint8_t* bt, bool fresh) {
-        const uint32_t aa = smem_u32(a), ba = smem_u32(bt);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t aoff = (uint32_t)(kk >> 2) * (kTile / 2) + (uint32_t)(kk & 3) * 32;
-          umma_f16(tmem_base + dcol, make_desc(aa + aoff, 16, 1024), make_desc(ba + (uint32_t)kk * 2048, kTile / 2, 1024),
-                   idesc_kmn, (fresh && kk == 0) ? 0u : 1u);
-        }
-      };
-      // D = A^T B with A a [k rows x m columns] tile and B a [k rows x n columns] tile, both read MN-major
-      auto mma_mnmn = [&](uint32_t dcol, const uint8_t* a, const uint8_t* bt) {
-        const uint32_t aa = smem_u32(a), ba = smem_u32(bt);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16(tmem_base + dcol, make_desc(aa + (uint32_t)kk * 2048, kTile / 2, 1024),
-                   make_desc(ba + (uint32_t)kk * 2048, kTile / 2, 1024), idesc_mnmn, kk != 0 ? 1u : 0u);
-      };
-      // Issue order per pair: dP^T, dV, then S^T of the NEXT pair (its TMEM columns are free once P^T has been formed, so
-      // the tensor core computes it while the warpgroups still work on dS^T), then dK and dQ.
-      bool ok = mbar_wait(kv_full, 0, abort_flag) && ring_wait(0);
+      __syncwarp();
+    } else if (warp == 13) {
+      // ------------------------------------------------------------ MMA issuer (the whole warp waits, one lane issues)
+      constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+      constexpr uint32_t idesc_kk = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+      constexpr uint32_t idesc_kmn = idesc_kk | (1u << 16);                 // B read MN-major
+      constexpr uint32_t idesc_mnmn = idesc_kk | (1u << 15) | (1u << 16);   // A and B read MN-major
+      const bool issuer = elect_one();
+      auto wait = [&](uint64_t* bar, int n) { return mbar_wait_warp(bar, (uint32_t)(n & 1), abort_flag); };
+      auto kdesc = [&](const uint8_t* tile) { return make_desc(smem_u32(tile), 16, 1024); };            // read K-major
+      auto mndesc = [&](const uint8_t* tile) { return make_desc(smem_u32(tile), kTile / 2, 1024); };    // read MN-major
+      const uint64_t dK_k = kdesc(sK), dV_k = kdesc(sV), dO_k = kdesc(sdO), dQ_k = kdesc(sQ), dS_k = kdesc(sS);
+      const uint64_t dK_mn = mndesc(sK), dO_mn = mndesc(sdO), dQ_mn = mndesc(sQ), dS_mn = mndesc(sS);
+      auto koff16 = [](int kk) { return (uint32_t)(((kk >> 2) * (kTile / 2) + (kk & 3) * 32) >> 4); };   // K-major: two 64-column atoms
+      auto mnoff16 = [](int kk) { return (uint32_t)((kk * 2048) >> 4); };                                // MN-major: 16 rows of 128 bytes
+      bool ok = n_it > 0 && wait(kv_full, 0) && wait(&q_full[0], 0);
       if (ok) {
         tc_fence_after();
-        mma_kk(kColS, sK, sR);                         // S^T of the first pair (ring item 0)
-        umma_commit(s_full);
-      }
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int nq = 2 * it, ndo = 2 * it + 1;
-        const uint32_t par = (uint32_t)(it & 1), prev = par ^ 1u;
-        const uint8_t* tQ = sR + (nq % kRing) * kTile;
-        const uint8_t* tdO = sR + (ndo % kRing) * kTile;
-        if (!ring_wait(ndo)) { ok = false; break; }
-        if (it > 0 && !mbar_wait(dq_drained, prev, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        mma_kk(kColDP, sV, tdO);                     // dP^T = V dO^T
-        umma_commit(dp_full);
-        if (!mbar_wait(p_ready, par, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        mma_kmn(kColDV, sP, tdO, it == 0);           // dV += P^T dO
-        if (it + 1 < n_it) {
-          if (!ring_wait(nq + 2)) { ok = false; break; }
-          if (!mbar_wait(s_free, par, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          mma_kk(kColS, sK, sR + ((nq + 2) % kRing) * kTile);   // S^T of the next pair
+        if (issuer) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) umma_f16(tmem_base + kColS, dK_k + koff16(kk), dQ_k + koff16(kk), idesc_kk, kk != 0 ? 1u : 0u);
           umma_commit(s_full);
         }
-        if (!mbar_wait(ds_ready, par, abort_flag)) { ok = false; break; }
+      }
+      for (int it = 0; it < n_it && ok; ++it) {
+        const uint32_t tq = (uint32_t)((it & 1) * (kTile >> 4)), tq_next = (uint32_t)(((it + 1) & 1) * (kTile >> 4));
+        if (!wait(do_full, it)) { ok = false; break; }
+        if (it > 0 && !wait(dq_drained, it - 1)) { ok = false; break; }
         tc_fence_after();
-        mma_kmn(kColDK, sS, tQ, it == 0);            // dK += dS^T Q
-        mma_mnmn(kColDP, sS, sK);                    // dQ = dS K (over the consumed dP^T)
-        umma_commit(mma2_done);
-        umma_commit(&r_empty[nq % kRing]);
-        umma_commit(&r_empty[ndo % kRing]);
+        if (issuer) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) umma_f16(tmem_base + kColDP, dV_k + koff16(kk), dO_k + koff16(kk), idesc_kk, kk != 0 ? 1u : 0u);
+          umma_commit(dp_full);                        // dP^T = V dO^T
+        }
+        if (!wait(p_ready, it)) { ok = false; break; }
+        tc_fence_after();
+        if (issuer) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)               // dV += P^T dO; P^T of 64 queries over the left of its half of S^T
+            umma_f16_ts(tmem_base + kColDV, tmem_base + kColS + (uint32_t)((kk >> 2) * 64 + (kk & 3) * 8), dO_mn + mnoff16(kk),
+                        idesc_kmn, (it == 0 && kk == 0) ? 0u : 1u);
+          umma_commit(do_empty);
+        }
+        if (it + 1 < n_it) {
+          if (!wait(&q_full[(it + 1) & 1], (it + 1) >> 1)) { ok = false; break; }
+          tc_fence_after();
+          if (issuer) {
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)             // S^T of the next pair, over P^T of this one
+              umma_f16(tmem_base + kColS, dK_k + koff16(kk), dQ_k + tq_next + koff16(kk), idesc_kk, kk != 0 ? 1u : 0u);
+            umma_commit(s_full);
+          }
+        }
+        if (!wait(ds_ready, it)) { ok = false; break; }
+        tc_fence_after();
+        if (issuer) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)               // dQ = dS K over the consumed dP^T
+            umma_f16(tmem_base + kColDP, dS_mn + mnoff16(kk), dK_mn + mnoff16(kk), idesc_mnmn, kk != 0 ? 1u : 0u);
+          umma_commit(dq_full);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)               // dK += dS^T Q
+            umma_f16(tmem_base + kColDK, dS_k + koff16(kk), dQ_mn + tq + mnoff16(kk), idesc_kmn, (it == 0 && kk == 0) ? 0u : 1u);
+          umma_commit(&q_empty[it & 1]);
+          if (it + 1 == n_it) umma_commit(all_done);
+        }
+      }
+      __syncwarp();
+    } else if (warp == 14) {
+      // ------------------------------------------------------------ lse (log2 domain, negated: an addend of the exponent) and
+      // delta (times the softmax scale, negated) of every query block; an lse of -inf switches a row off
+      // (read one block ahead, all eight loads in flight at once)
+      int h = hk * G, i = 0;
+      float l[4], d[4];
+      auto fetch = [&]() {
+        const int64_t base = p.cu_q ? (int64_t)h * p.total_q + qoff : ((int64_t)b * p.H + h) * p.Sq;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int qi = (i0 + i) * BQ + e * 32 + lane;
+          l[e] = qi < Sq ? __ldg(p.lse + base + qi) : -INFINITY;
+          d[e] = qi < Sq ? __ldg(p.delta + base + qi) : 0.f;
+        }
+      };
+      if (n_it > 0) fetch();
+      for (int it = 0; it < n_it; ++it) {
+        const int st = it & 1;
+        if (!mbar_wait_warp(&ld_empty[st], (uint32_t)(((it >> 1) & 1) ^ 1), abort_flag)) break;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s_lse[st * 128 + e * 32 + lane] = l[e] > -INFINITY ? -l[e] * 1.4426950408889634f : -INFINITY;
+          s_dlt[st * 128 + e * 32 + lane] = -d[e] * p.scale;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ld_full[st]);
+        if (++i == n_i) { i = 0; ++h; }
+        if (it + 1 < n_it) fetch();
       }
     }
-    __syncwarp();
+  } else if (warp >= 8) {
+    regs_inc<kDqRegs>();
+    // ------------------------------------------------------------ dQ warpgroup: TMEM -> registers -> shared memory -> global
+    const int qw = warp & 3;
+    const int r = qw * 32 + lane;                 // query row inside the block = TMEM lane
+    const uint32_t addr = tmem_base + ((uint32_t)(qw * 32) << 16) + kColDP;
+    int h = hk * G, i = 0;
+    for (int it = 0; it < n_it; ++it) {
+      const int q0 = (i0 + i) * BQ;
+      bool ok = mbar_wait_warp(dq_full, (uint32_t)(it & 1), abort_flag);
+      tc_fence_after();
+      uint32_t raw[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld32(addr + (uint32_t)(c * 32), raw[c]);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(dq_drained);
+      const int row0 = p.cu_q ? (int)((int64_t)h * p.total_q + qoff + q0) : (int)(((int64_t)b * p.H + h) * p.Sq + q0);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        // the reduction that read this box two chunks ago has finished with it
+        if (threadIdx.x == 8 * 32) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        if (!named_bar_and(1, 128, ok)) { ok = false; break; }     // one answer for the four warps
+        uint8_t* box = sStage + (c & 1) * kStage + (size_t)r * 128;
+#pragma unroll
+        for (int ch = 0; ch < 8; ++ch)
+          *reinterpret_cast<uint4*>(box + (size_t)((ch ^ (r & 7)) * 16)) =
+              make_uint4(raw[c][ch * 4], raw[c][ch * 4 + 1], raw[c][ch * 4 + 2], raw[c][ch * 4 + 3]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        named_bar_sync(1, 128);
+        if (threadIdx.x == 8 * 32) {
+          tma_reduce_add_2d(&tmap_dq, sStage + (c & 1) * kStage, c * 32, row0);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+      if (!ok) break;
+      if (++i == n_i) { i = 0; ++h; }
+    }
+    // every reduction must have completed before the CTA exits
+    if (threadIdx.x == 8 * 32) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   } else {
+    regs_inc<kComputeRegs>();
     // ------------------------------------------------------------ two compute warpgroups (warps 0-3, 4-7)
     const int wg = warp >> 2;
     const int qw = warp & 3;
     const int r = qw * 32 + lane;                 // key row inside the block = TMEM lane
     const int kj = k0 + r;
     const uint32_t lane_base = ((uint32_t)(qw * 32) << 16);
-    const int tid = threadIdx.x;                  // 0..255 here
-    uint8_t* prow = sP + (size_t)wg * (kTile / 2) + (size_t)r * 128;   // this warpgroup's 64 query columns = atom `wg`
-    uint8_t* srow = sS + (size_t)wg * (kTile / 2) + (size_t)r * 128;
+    const uint32_t s_addr = tmem_base + lane_base + kColS + (uint32_t)(wg * 64);
+    const uint32_t dp_addr = tmem_base + lane_base + kColDP + (uint32_t)(wg * 64);
+    uint8_t* srow = sS + (size_t)wg * (kTile / 2) + (size_t)r * 128;   // this warpgroup's 64 query columns = atom `wg`
+    const bool key_off = kj >= Sk;
+    const bool block_off = k0 + BK > Sk;
     bool ok = true;
-    auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-      const bool w = mbar_wait(bar, parity, abort_flag);
-      return __all_sync(0xffffffffu, w);
-    };
+    auto wait_all = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity, abort_flag); };
+    int i = 0;
     for (int it = 0; it < n_it; ++it) {
       const uint32_t par = (uint32_t)(it & 1);
-      const int h = hk * G + it / n_i;
-      const int q0 = (i0 + it % n_i) * BQ;
-      // lse (log2 domain) and delta (times the softmax scale) of the 128 query rows of this block; +inf switches a row
-      // off.  Single buffers: a thread gets here only after mma2_done of the previous pair, which needs every warp's
-      // ds_ready, i.e. all reads of the previous values.
-      {
-        const int which = tid >> 7, q = tid & 127, qi = q0 + q;
-        const int64_t idx = p.cu_q ? (int64_t)h * p.total_q + qoff + qi : ((int64_t)b * p.H + h) * p.Sq + qi;
-        if (which == 0) {
-          float l = qi < Sq ? p.lse[idx] : -INFINITY;
-          s_lse[q] = l > -INFINITY ? -l * 1.4426950408889634f : -INFINITY;   // negated: an addend of the exponent
-        } else {
-          s_dlt[q] = qi < Sq ? -p.delta[idx] * p.scale : 0.f;              // negated and scaled likewise
-        }
-      }
-      named_bar_sync(1, 256);
-      const float4* nlse4 = reinterpret_cast<const float4*>(s_lse + wg * 64);
-      const float4* ndlt4 = reinterpret_cast<const float4*>(s_dlt + wg * 64);
-      const bool diag = p.causal && q0 < k0 + BK;       // only then can a query be older than a key of this block
-      const bool key_off = kj >= Sk;
-      if (!wait_all(s_full, par)) { ok = false; break; }
-      // the staged dQ of the previous pair must have left the shared memory that P^T is written to
-      if (it > 0 && !wait_all(stage_free, par ^ 1u)) { ok = false; break; }
+      const int st = it & 1, q0 = (i0 + i) * BQ;
+      const float4* nlse4 = reinterpret_cast<const float4*>(s_lse + st * 128 + wg * 64);
+      const float4* ndlt4 = reinterpret_cast<const float4*>(s_dlt + st * 128 + wg * 64);
+      // only then can a query be older than a key of this block, or a key be past the end
+      const bool masked = (p.causal && q0 < k0 + BK) || block_off;
+      if (!wait_all(&ld_full[st], (uint32_t)((it >> 1) & 1)) || !wait_all(s_full, par)) { ok = false; break; }
       tc_fence_after();
       float pf[64];
-      {
-        uint32_t ra[32], rb[32];
-        auto chunk_p = [&](const uint32_t (&raw)[32], int c) {
-          uint32_t pk[16];
+      auto probs = [&](auto mask) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t raw[32], pk[16];
+          tmem_ld32(s_addr + (uint32_t)(c * 32), raw);
+          tmem_ld_wait();
 #pragma unroll
           for (int e4 = 0; e4 < 8; ++e4) {
             const float4 nl = nlse4[c * 8 + e4];
@@ -293,116 +374,64 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
               float x0, x1;
               fma2v(x0, x1, __uint_as_float(raw[e]), __uint_as_float(raw[e + 1]), p.scale_log2, nls[e2], nls[e2 + 1]);
               float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
-              if (key_off || diag) {
+              if constexpr (decltype(mask)::value) {
                 const int qi = q0 + wg * 64 + cc;
-                if (key_off || qi < kj) p0 = 0.f;
-                if (key_off || qi + 1 < kj) p1 = 0.f;
+                if (key_off || (p.causal && qi < kj)) p0 = 0.f;
+                if (key_off || (p.causal && qi + 1 < kj)) p1 = 0.f;
               }
               pf[cc] = p0;
               pf[cc + 1] = p1;
               pk[e >> 1] = pack2<T>(p0, p1);
             }
           }
+          tmem_st16(s_addr + (uint32_t)(c * 16), pk);   // over columns of S^T that this thread has read
+        }
+      };
+      if (masked) probs(std::true_type{});
+      else probs(std::false_type{});
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_ready);
+      // dP^T; its commit also says that the products which read the previous dS^T have completed
+      if (!wait_all(dp_full, par)) { ok = false; break; }
+      tc_fence_after();
 #pragma unroll
-          for (int g8 = 0; g8 < 4; ++g8) {
-            const int ch = c * 4 + g8;
-            *reinterpret_cast<uint4*>(prow + (size_t)((ch ^ (r & 7)) * 16)) =
-                make_uint4(pk[g8 * 4], pk[g8 * 4 + 1], pk[g8 * 4 + 2], pk[g8 * 4 + 3]);
+      for (int c = 0; c < 2; ++c) {
+        uint32_t raw[32], pk[16];
+        tmem_ld32(dp_addr + (uint32_t)(c * 32), raw);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e4 = 0; e4 < 8; ++e4) {
+          const float4 nd = ndlt4[c * 8 + e4];
+          const float nds[4] = {nd.x, nd.y, nd.z, nd.w};
+#pragma unroll
+          for (int e2 = 0; e2 < 4; e2 += 2) {
+            const int e = e4 * 4 + e2, cc = c * 32 + e;
+            float t0, t1, d0, d1;
+            fma2v(t0, t1, __uint_as_float(raw[e]), __uint_as_float(raw[e + 1]), p.scale, nds[e2], nds[e2 + 1]);
+            mul2(d0, d1, pf[cc], pf[cc + 1], t0, t1);
+            pk[e >> 1] = pack2<T>(d0, d1);
           }
-        };
-        const uint32_t addr = tmem_base + lane_base + kColS + (uint32_t)(wg * 64);
-        tmem_ld32(addr, ra);
-        tmem_ld_wait();
-        tmem_ld32(addr + 32u, rb);
-        chunk_p(ra, 0);
-        tmem_ld_wait();
-        chunk_p(rb, 1);
+        }
+#pragma unroll
+        for (int g8 = 0; g8 < 4; ++g8) {
+          const int ch = c * 4 + g8;
+          *reinterpret_cast<uint4*>(srow + (size_t)((ch ^ (r & 7)) * 16)) =
+              make_uint4(pk[g8 * 4], pk[g8 * 4 + 1], pk[g8 * 4 + 2], pk[g8 * 4 + 3]);
+        }
       }
       tc_fence_before();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(s_free);
-        mbar_arrive(p_ready);
+        mbar_arrive(ds_ready);
+        mbar_arrive(&ld_empty[st]);
       }
-      if (!wait_all(dp_full, par)) { ok = false; break; }
-      tc_fence_after();
-      {
-        uint32_t ra[32], rb[32];
-        auto chunk_ds = [&](const uint32_t (&raw)[32], int c) {
-          uint32_t pk[16];
-#pragma unroll
-          for (int e4 = 0; e4 < 8; ++e4) {
-            const float4 nd = ndlt4[c * 8 + e4];
-            const float nds[4] = {nd.x, nd.y, nd.z, nd.w};
-#pragma unroll
-            for (int e2 = 0; e2 < 4; e2 += 2) {
-              const int e = e4 * 4 + e2, cc = c * 32 + e;
-              float t0, t1, d0, d1;
-              fma2v(t0, t1, __uint_as_float(raw[e]), __uint_as_float(raw[e + 1]), p.scale, nds[e2], nds[e2 + 1]);
-              mul2(d0, d1, pf[cc], pf[cc + 1], t0, t1);
-              pk[e >> 1] = pack2<T>(d0, d1);
-            }
-          }
-#pragma unroll
-          for (int g8 = 0; g8 < 4; ++g8) {
-            const int ch = c * 4 + g8;
-            *reinterpret_cast<uint4*>(srow + (size_t)((ch ^ (r & 7)) * 16)) =
-                make_uint4(pk[g8 * 4], pk[g8 * 4 + 1], pk[g8 * 4 + 2], pk[g8 * 4 + 3]);
-          }
-        };
-        const uint32_t addr = tmem_base + lane_base + kColDP + (uint32_t)(wg * 64);
-        tmem_ld32(addr, ra);
-        tmem_ld_wait();
-        tmem_ld32(addr + 32u, rb);
-        chunk_ds(ra, 0);
-        tmem_ld_wait();
-        chunk_ds(rb, 1);
-      }
-      tc_fence_before();
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(ds_ready);
-      // dQ of this pair: lane = query row, this warpgroup's 64 head-dim columns.  Staged as fp32 in the 64 KB that
-      // P^T and dS^T occupied (the MMAs that read them have completed): four [128 rows x 128 bytes] boxes, 128B-swizzled.
-      if (!wait_all(mma2_done, par)) { ok = false; break; }
-      tc_fence_after();
-      {
-        uint32_t ra[32], rb[32];
-        auto stage = [&](const uint32_t (&raw)[32], int c) {
-          uint8_t* box = sP + (size_t)(wg * 2 + c) * (kTile / 2) + (size_t)r * 128;
-#pragma unroll
-          for (int ch = 0; ch < 8; ++ch)
-            *reinterpret_cast<uint4*>(box + (size_t)((ch ^ (r & 7)) * 16)) =
-                make_uint4(raw[ch * 4], raw[ch * 4 + 1], raw[ch * 4 + 2], raw[ch * 4 + 3]);
-        };
-        const uint32_t addr = tmem_base + lane_base + kColDP + (uint32_t)(wg * 64);
-        tmem_ld32(addr, ra);
-        tmem_ld_wait();
-        tmem_ld32(addr + 32u, rb);
-        stage(ra, 0);
-        tmem_ld_wait();
-        stage(rb, 1);
-      }
-      tc_fence_before();
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dq_drained);
-      named_bar_sync(2, 256);
-      if (tid == 0) {
-        const int row0 = p.cu_q ? (int)((int64_t)h * p.total_q + qoff + q0) : (int)(((int64_t)b * p.H + h) * p.Sq + q0);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          tma_reduce_add_2d(&tmap_dq, sP + (size_t)c * (kTile / 2), c * 32, row0);
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        mbar_arrive(stage_free);
-      }
-      __syncwarp();
+      if (++i == n_i) i = 0;
     }
-    // every reduction must have completed before the CTA exits
-    if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-    // ---- dK, dV of this key block (all pairs have completed: the last mma2_done was waited for above)
+    if (ok && n_it > 0) ok = wait_all(all_done, 0);
+    // ---- dK, dV of this key block
     if (ok) {
       tc_fence_after();
       const bool row_ok = kj < Sk;
@@ -435,9 +464,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
   }
 
+  // a CTA that gave up on a wait may still have tile loads in flight towards its shared memory: give them a bounded moment
+  if (*abort_flag && threadIdx.x == 0)
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == 13) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kBwdTmemCols);
   }
@@ -464,27 +496,57 @@ bool make_dq_map(CUtensorMap* out, float* ptr, int64_t rows) {
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// delta[b, h, q] = sum_d O[b, h, q, d] * dO[b, h, q, d]; one warp per row
+// delta[b, h, q] = sum_d O[b, h, q, d] * dO[b, h, q, d], and the row of the fp32 dQ buffer is zeroed on the way.  Sixteen
+// lanes per row with 16-byte accesses, 64 consecutive rows of one (batch, head) per block, four rows in flight per lane:
+// bound by memory (2 x 256 bytes in, 512 out per row).  32 x 4096 rows: 24 us, against 30 (8-byte loads, a row per warp,
+// 64-bit divisions for its place) + 11 for the memset it replaces.
+constexpr int kDeltaRows = 64;
 template <typename T>
-__global__ void attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ d_o, float* __restrict__ delta, int B,
-                                  int H, int Sq, int64_t o_sb, int64_t o_sh, int64_t o_ss, int64_t g_sb, int64_t g_sh,
-                                  int64_t g_ss) {
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= (int64_t)B * H * Sq) return;
-  const int q = (int)(row % Sq);
-  const int h = (int)((row / Sq) % H);
-  const int b = (int)(row / ((int64_t)Sq * H));
-  const T* po = o + b * o_sb + h * o_sh + q * o_ss + lane * 4;
-  const T* pg = d_o + b * g_sb + h * g_sh + q * g_ss + lane * 4;
-  const uint2 a = *reinterpret_cast<const uint2*>(po), g = *reinterpret_cast<const uint2*>(pg);
-  const T* av = reinterpret_cast<const T*>(&a);
-  const T* gv = reinterpret_cast<const T*>(&g);
-  float s = 0.f;
+__global__ void __launch_bounds__(256) attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ d_o, float* __restrict__ delta,
+                                                         float* __restrict__ dq, int H, int Sq, int row_blocks, int64_t o_sb,
+                                                         int64_t o_sh, int64_t o_ss, int64_t g_sb, int64_t g_sh, int64_t g_ss) {
+  const int bh = (int)(blockIdx.x / row_blocks);
+  const int b = bh / H, h = bh - b * H;
+  const int q0 = (int)(blockIdx.x - (unsigned)bh * row_blocks) * kDeltaRows + (threadIdx.x >> 4);
+  const int l16 = threadIdx.x & 15;
+  const T* po = o + b * o_sb + h * o_sh + l16 * 8;
+  const T* pg = d_o + b * g_sb + h * g_sh + l16 * 8;
+  Vec16<T> av[4], gv[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) s += ToF<T>::to(av[e]) * ToF<T>::to(gv[e]);
-  s = warp_sum(s);
-  if (lane == 0) delta[row] = s;
+  for (int i = 0; i < 4; ++i) {
+    const int q = q0 + i * 16;
+    if (q < Sq) {
+      av[i] = ld16(po + q * o_ss);
+      gv[i] = ld16(pg + q * g_ss);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int q = q0 + i * 16;
+    float s = 0.f;
+    if (q < Sq) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s += ToF<T>::to(av[i].v[e]) * ToF<T>::to(gv[i].v[e]);
+    }
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1) s += __shfl_xor_sync(0xffffffffu, s, w);
+    if (q < Sq) {
+      const int64_t row = (int64_t)bh * Sq + q;
+      if (l16 == 0) delta[row] = s;
+      float4* z = reinterpret_cast<float4*>(dq + row * BD);
+      z[l16] = make_float4(0.f, 0.f, 0.f, 0.f);
+      z[l16 + 16] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+}
+
+template <typename K>
+int bwd_setup(K kern) {
+  cudaFuncAttributes at;
+  cudaError_t e = cudaFuncGetAttributes(&at, kern);
+  if (e != cudaSuccess) return (int)e;
+  if (at.numRegs < kLaunchRegs) return (int)cudaErrorNotSupported;   // the register split would wait for ever
+  return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
 }
 
 }  // namespace
@@ -550,30 +612,21 @@ extern "C" int b200_flash_attn_bwd(const b200_attn_t* a, float* dq_accum, void* 
   p.total_q = a->total_q;
   const long long grid = (long long)a->B * a->Hkv * p.kv_blocks;
   if (grid > 2147483647ll || rows / 8 + 1 > 2147483647ll) return (int)cudaErrorNotSupported;
-  cudaError_t e = cudaMemsetAsync(dq_accum, 0, (size_t)rows * BD * sizeof(float), stream);
-  if (e != cudaSuccess) return (int)e;
+  const int row_blocks = (dS + kDeltaRows - 1) / kDeltaRows;
+  const unsigned delta_grid = (unsigned)((long long)dB * a->H * row_blocks);
   if (bf16) {
-    attn_delta_kernel<__nv_bfloat16><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(
-        (const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, dB, a->H, dS, a->o_sb, a->o_sh, a->o_ss, x[0], x[1], x[2]);
-    static bool set = false;
-    auto kern = attn_bwd_kernel<__nv_bfloat16>;
-    if (!set) {
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
-      if (e != cudaSuccess) return (int)e;
-      set = true;
-    }
-    kern<<<(unsigned)grid, kBwdThreads, kBwdSmem, stream>>>(mq, mk, mv, mdo, mdq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, p);
+    static const int setup = bwd_setup(attn_bwd_kernel<__nv_bfloat16>);
+    if (setup != 0) return setup;
+    attn_delta_kernel<__nv_bfloat16><<<delta_grid, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, dq_accum,
+                                                                     a->H, dS, row_blocks, a->o_sb, a->o_sh, a->o_ss, x[0], x[1], x[2]);
+    attn_bwd_kernel<__nv_bfloat16><<<(unsigned)grid, kBwdThreads, kBwdSmem, stream>>>(mq, mk, mv, mdo, mdq, (__nv_bfloat16*)dk,
+                                                                                     (__nv_bfloat16*)dv, p);
   } else {
-    attn_delta_kernel<__half><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(
-        (const __half*)o, (const __half*)d_o, delta, dB, a->H, dS, a->o_sb, a->o_sh, a->o_ss, x[0], x[1], x[2]);
-    static bool set = false;
-    auto kern = attn_bwd_kernel<__half>;
-    if (!set) {
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
-      if (e != cudaSuccess) return (int)e;
-      set = true;
-    }
-    kern<<<(unsigned)grid, kBwdThreads, kBwdSmem, stream>>>(mq, mk, mv, mdo, mdq, (__half*)dk, (__half*)dv, p);
+    static const int setup = bwd_setup(attn_bwd_kernel<__half>);
+    if (setup != 0) return setup;
+    attn_delta_kernel<__half><<<delta_grid, 256, 0, stream>>>((const __half*)o, (const __half*)d_o, delta, dq_accum, a->H, dS, row_blocks,
+                                                              a->o_sb, a->o_sh, a->o_ss, x[0], x[1], x[2]);
+    attn_bwd_kernel<__half><<<(unsigned)grid, kBwdThreads, kBwdSmem, stream>>>(mq, mk, mv, mdo, mdq, (__half*)dk, (__half*)dv, p);
   }
   note_launch(2);
   return (int)cudaGetLastError();
