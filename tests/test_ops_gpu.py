@@ -374,3 +374,62 @@ def test_swiglu_limited_to_live_rows(bw, dev):
     gr, ur = xr.chunk(2, -1)
     (torch.nn.functional.silu(gr) * ur)[:live].backward(dy.float()[:live])
     assert (xd.grad[:live].float().cpu() - xr.grad[:live]).abs().max() < 3e-2
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 1000), (297, 2048), (1300, 4096), (40, 8192), (7, 16384), (301, 24576), (2, 32768), (5, 4100)])
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("with_residual_grad", [True, False])
+def test_rms_norm_residual_backward(bw, dev, rows, cols, dt, with_residual_grad):
+    """Every ring depth of the backward (four slots, fewer for wide rows, one for the widest), strips of several rows, the
+    widths that keep a row in registers and those that read it twice; 4100 columns of 16 bits take the general route."""
+    from torch_musa_b200.ops import rms_norm_residual
+
+    if cols * (4 if dt == torch.float32 else 2) > 65536:
+        pytest.skip("wider than the forward kernel takes")
+    torch.manual_seed(rows + cols)
+    if cols % (4 if dt == torch.float32 else 8):
+        op = lambda *a: torch.ops.blackwell.rms_norm_residual_backward(*a)   # the forward has no general route
+        res, dy, dres, w = (torch.randn(s).to(dt) for s in ((rows, cols), (rows, cols), (rows, cols), (cols,)))
+        rstd = torch.rsqrt(res.double().square().mean(-1, keepdim=True) + 1e-5).float()
+        dx, dw = op(dy.to(dev), dres.to(dev) if with_residual_grad else None, res.to(dev), rstd.to(dev), w.to(dev))
+    else:
+        x, r, dy, dres, w = (torch.randn(s).to(dt) for s in ((rows, cols), (rows, cols), (rows, cols), (rows, cols), (cols,)))
+        xd, rd, wd = (t.to(dev).requires_grad_() for t in (x, r, w))
+        y, h = rms_norm_residual(xd, rd, wd, 1e-5)
+        outs, gs = ([y, h], [dy.to(dev), dres.to(dev)]) if with_residual_grad else ([y], [dy.to(dev)])
+        dx, dr, dw = torch.autograd.grad(outs, [xd, rd, wd], gs)
+        assert torch.equal(dx.cpu(), dr.cpu())
+        res = h.detach().cpu()
+    rs = res.double().requires_grad_()
+    wr = w.double().requires_grad_()
+    F.rms_norm(rs, (cols,), wr, 1e-5).backward(dy.double())
+    want = rs.grad + (dres.double() if with_residual_grad else 0)
+    # sums of `cols` (dx) and `rows` (dw) fp32 terms, then one rounding to the type: covered by the type's tolerance
+    assert close(dx, want, dt) and close(dw, wr.grad, dt)
+    bw.synchronize()
+    assert bw._C._gemm_status(False) == 0
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (5, 4001), (700, 520), (1300, 4104), (1200, 32000)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_fused_cross_entropy_row_widths(bw, dev, rows, cols, dt):
+    """Each number of threads per row, remainders of the four-vector loads, rows with -inf entries, and no target that
+    counts at all."""
+    from torch_musa_b200.ops import fused_cross_entropy
+
+    torch.manual_seed(rows)
+    x = (torch.randn(rows, cols) * 3).to(dt)
+    if cols > 8:
+        x[:, 3] = float("-inf")
+    t = torch.randint(4, cols, (rows,))
+    t[1::5] = -100
+    xd, xr = x.to(dev).requires_grad_(), x.double().requires_grad_()
+    loss = fused_cross_entropy(xd, t.to(dev))
+    loss.backward()
+    ref = F.cross_entropy(xr, t)
+    ref.backward()
+    assert abs(float(loss) - float(ref)) < 2e-6 * max(1.0, abs(float(ref))) * 4     # fp32 sums, fast exponentials (2^-21)
+    lim = {torch.float32: 2e-6, torch.bfloat16: 2.0 ** -8}[dt]
+    assert float((xd.grad.double().cpu() - xr.grad).abs().max()) <= lim * float(xr.grad.abs().max())
+    none = fused_cross_entropy(x.to(dev), torch.full((rows,), -100).to(dev))
+    assert float(none) == 0.0

@@ -226,6 +226,60 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rms_norm_residual(const at::Tenso
   return {y, res, rstd};
 }
 
+// Gradients of rms_norm_residual: dx (= the gradient of x and of the residual), with the gradient dres of the sum added
+// inside the kernel, and dw.
+std::tuple<at::Tensor, at::Tensor> rms_norm_residual_backward(const at::Tensor& dy, const std::optional<at::Tensor>& dres,
+                                                              const at::Tensor& res, const at::Tensor& rstd,
+                                                              const at::Tensor& weight) {
+  check_fast(res, "rms_norm_residual_backward");
+  check_devices("rms_norm_residual_backward", res, dy, rstd, weight);
+  const bool has_dres = dres.has_value() && dres->defined();
+  if (has_dres) check_devices("rms_norm_residual_backward", res, *dres);
+  const int64_t cols = res.size(-1), rows = cols ? res.numel() / cols : 0;
+  if (rows > 0 && dy.scalar_type() == res.scalar_type() && weight.scalar_type() == res.scalar_type() &&
+      dy.sizes() == res.sizes() && rstd.scalar_type() == at::kFloat && rstd.numel() == rows &&
+      (!has_dres || (dres->scalar_type() == res.scalar_type() && dres->sizes() == res.sizes()))) {
+    at::Tensor x = res.contiguous(), g = dy.contiguous(), w = weight.contiguous(), rs = rstd.contiguous(), r;
+    if (has_dres) r = dres->contiguous();
+    at::Tensor dx = at::empty_like(x), dw = at::empty_like(w);
+    const int nb = b200_rmsnorm_bwd_partial_rows(rows, cols);
+    at::Tensor partial = at::empty({nb, cols}, x.options().dtype(at::kFloat));
+    DeviceSwitch sw(x.device().index());
+    cudaStream_t s = current_raw_stream(x);
+    const int err = b200_rmsnorm_bwd(kdtype(x.scalar_type()), dx.mutable_data_ptr(), partial.data_ptr<float>(), nullptr,
+                                     g.const_data_ptr(), x.const_data_ptr(), w.const_data_ptr(), rs.data_ptr<float>(),
+                                     has_dres ? r.const_data_ptr() : nullptr, rows, cols, s);
+    if (err == 0) {
+      B200_KERNEL_CALL(b200_reduce_cols_sum(B200_F32, dw.mutable_data_ptr(), kdtype(dw.scalar_type()), partial.const_data_ptr(),
+                                            nb, cols, s));
+      return {dx, dw};
+    }
+    if (err != (int)cudaErrorNotSupported) B200_KERNEL_CALL(err);
+  }
+  auto [dx, dw] = at::_fused_rms_norm_backward(dy.contiguous(), res, {cols}, rstd, weight, {true, true});
+  return {has_dres ? at::add(dx, *dres) : dx, dw};
+}
+
+// (mean over the counted rows, their number): what reduction="mean" makes of the row losses, in one launch.
+std::tuple<at::Tensor, at::Tensor> cross_entropy_mean(const at::Tensor& loss_rows, const at::Tensor& target,
+                                                      int64_t ignore_index) {
+  check_fast(loss_rows, "cross_entropy_mean");
+  check_devices("cross_entropy_mean", loss_rows, target);
+  TORCH_CHECK(loss_rows.dim() == 1 && loss_rows.scalar_type() == at::kFloat && target.dim() == 1 &&
+                  target.size(0) == loss_rows.size(0) && target.scalar_type() == at::kLong && on_device(target),
+              "cross_entropy_mean: expected float32 losses [T] and int64 targets [T] on the device");
+  if (loss_rows.numel() == 0 || loss_rows.numel() > 65536) {   // one block adds up to 64 rows per thread
+    at::Tensor n = target.ne(ignore_index).sum().clamp_min(1).to(at::kFloat);
+    return {at::div(loss_rows.sum(), n), n};
+  }
+  at::Tensor l = loss_rows.contiguous(), t = target.contiguous();
+  at::Tensor mean = at::empty({}, l.options()), count = at::empty({}, l.options());
+  DeviceSwitch sw(l.device().index());
+  B200_KERNEL_CALL(b200_cross_entropy_mean(mean.data_ptr<float>(), count.data_ptr<float>(), l.data_ptr<float>(),
+                                           t.data_ptr<int64_t>(), l.numel(), ignore_index, current_raw_stream(l)));
+  return {mean, count};
+}
+
 at::Tensor decode_attention(const at::Tensor& q, const at::Tensor& k_cache, const at::Tensor& v_cache,
                             const at::Tensor& pos, std::optional<double> scale) {
   check_fast(q, "decode_attention");
@@ -358,6 +412,8 @@ TORCH_LIBRARY(blackwell, m) {
   m.def("online_softmax_stats(Tensor logits, Tensor target, int vocab_start) -> Tensor");
   m.def("vocab_parallel_ce_finish(Tensor(a!) logits, Tensor all_stats, Tensor target, int vocab_start, int ignore_index) -> Tensor");
   m.def("rms_norm_residual(Tensor x, Tensor residual, Tensor weight, float eps) -> (Tensor, Tensor, Tensor)");
+  m.def("rms_norm_residual_backward(Tensor dy, Tensor? dres, Tensor res, Tensor rstd, Tensor weight) -> (Tensor, Tensor)");
+  m.def("cross_entropy_mean(Tensor loss_rows, Tensor target, int ignore_index=-100) -> (Tensor, Tensor)");
   m.def("multi_tensor_l2norm(Tensor[] tensors, bool per_tensor=False) -> (Tensor, Tensor)");
   m.def("multi_tensor_scale_(Tensor(a!)[] tensors, Tensor? inv_scale, float scale, Tensor(b!) found_inf) -> ()");
   m.def("multi_tensor_axpby_(Tensor(a!)[] out, Tensor[] x, Tensor[] y, float a, float b) -> ()");
@@ -387,6 +443,8 @@ TORCH_LIBRARY_IMPL(blackwell, PrivateUse1, m) {
   m.impl("online_softmax_stats", TORCH_FN(online_softmax_stats));
   m.impl("vocab_parallel_ce_finish", TORCH_FN(vocab_parallel_ce_finish));
   m.impl("rms_norm_residual", TORCH_FN(rms_norm_residual));
+  m.impl("rms_norm_residual_backward", TORCH_FN(rms_norm_residual_backward));
+  m.impl("cross_entropy_mean", TORCH_FN(cross_entropy_mean));
 }
 
 TORCH_LIBRARY_IMPL(blackwell, CompositeExplicitAutograd, m) { m.impl("_sleep", TORCH_FN(sleep_cycles)); }

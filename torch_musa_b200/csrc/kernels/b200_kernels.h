@@ -205,8 +205,8 @@ B200_API int b200_rmsnorm_fwd(int dtype, void* y, float* rstd, const void* x, co
                               void* res_out, int64_t rows, int64_t cols, float eps, cudaStream_t stream);
 /* dx (and optionally dw partial sums in dw_partial[nblocks, cols] fp32; pass NULL to skip) */
 B200_API int b200_rmsnorm_bwd(int dtype, void* dx, float* dw_partial, int* nblocks_out_host, const void* dy,
-                              const void* x, const void* w, const float* rstd, int64_t rows, int64_t cols,
-                              cudaStream_t stream);
+                              const void* x, const void* w, const float* rstd, const void* dres /* added to dx, may be
+                              NULL */, int64_t rows, int64_t cols, cudaStream_t stream);
 B200_API int b200_rmsnorm_bwd_partial_rows(int64_t rows, int64_t cols);
 B200_API int b200_layernorm_fwd(int dtype, void* y, float* mean, float* rstd, const void* x, const void* w,
                                 const void* b, int64_t rows, int64_t cols, float eps, cudaStream_t stream);
@@ -225,6 +225,9 @@ B200_API int b200_cross_entropy_fwd(int dtype, float* loss, float* lse, const vo
                                     int64_t rows, int64_t cols, int64_t ignore_index, float label_smoothing,
                                     cudaStream_t stream);
 /* dlogits = (softmax - onehot) * grad_scale[row or scalar]; may run in place over logits */
+/* mean[0] = sum of loss over the rows / max(1, number of targets that are not ignore_index), count[0] = that number */
+B200_API int b200_cross_entropy_mean(float* mean, float* count, const float* loss, const int64_t* target, int64_t rows,
+                                     int64_t ignore_index, cudaStream_t stream);
 B200_API int b200_cross_entropy_bwd(int dtype, void* dlogits, const void* logits, const float* lse,
                                     const int64_t* target, const float* grad_loss, int grad_is_scalar, float scale,
                                     int64_t rows, int64_t cols, int64_t ignore_index, float label_smoothing,

@@ -6,10 +6,21 @@
 // the caller reduces with the column-sum kernel (deterministic, no atomics).
 // Parity: reference torch_musa/csrc/aten/ops/RMSNorm.cpp:113-125,283-306 and
 // LayerNorm.cpp:141-147,295-300 (vendor-library calls there).
-#include "common.cuh"
+#include "gemm_common.cuh"   // mbarriers
+
+#include <algorithm>
 
 namespace b200k {
 namespace {
+
+constexpr int kMaxRmsStages = 4;
+
+// contiguous bytes from global to shared memory, credited to the barrier (16-byte aligned, a multiple of 16 bytes)
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(gemmdev::smem_u32(dst)), "l"(src), "r"(bytes), "r"(gemmdev::smem_u32(bar))
+               : "memory");
+}
 
 
 template <typename T, int THREADS, int VPT>
@@ -62,73 +73,155 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_fwd_kernel(T* __restrict__ y,
   }
 }
 
-// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)), xhat = x*rstd. A CTA walks a strip of rows and keeps
-// dw partial sums (dy * xhat) for its columns in registers.
+// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres), xhat = x*rstd. A CTA walks a strip of rows and keeps
+// dw partial sums (dy * xhat) for its columns in registers.  dres is the gradient that reaches the row past the norm (a
+// residual stream): adding it here saves a pass over three tensors.
+//
+// A row's dot product stands between its loads and its stores, so rows come through a ring of `stages` slots in shared
+// memory (x, dy, dres of a row each), filled by bulk copies several rows ahead: bound by memory then, not by its latency.
+// One barrier per row serves the reduction (its partial sums alternate between two buffers) and says that the slot
+// has been read, so thread 0 refills it.  Waits are bounded; a block that gave up leaves as a whole and sets the status.
+// 4096 x 4096 bf16 with dres: 60.5 us as two kernels before (44.6 + 15.9), 26.6 now (5.0 TB/s).
+struct RmsBwdParams {
+  int64_t rows, cols;
+  int rows_per_cta, stages;
+  int* status;
+};
+
 template <typename T, int THREADS, int VPT>
 __global__ void __launch_bounds__(THREADS) rmsnorm_bwd_kernel(T* __restrict__ dx, float* __restrict__ dw_partial,
                                                               const T* __restrict__ dy, const T* __restrict__ x,
                                                               const T* __restrict__ w, const float* __restrict__ rstd,
-                                                              int64_t rows, int64_t cols, int rows_per_cta) {
+                                                              const T* __restrict__ dres, const RmsBwdParams p) {
+  using namespace gemmdev;
   constexpr int V = Vec16<T>::N;
-  __shared__ float sh[32];
+  extern __shared__ __align__(16) uint8_t ring[];
+  __shared__ float sh[2][32];
+  __shared__ uint64_t full[kMaxRmsStages];
+  __shared__ int abort_word;
+  volatile int* abort_flag = &abort_word;
+  const int64_t cols = p.cols;
   const int nvec = (int)(cols / V);
+  const uint32_t row_bytes = (uint32_t)(cols * sizeof(T));
+  const int tensors = dres ? 3 : 2;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t r0 = (int64_t)blockIdx.x * p.rows_per_cta;
+  const int n = (int)(min(r0 + (int64_t)p.rows_per_cta, p.rows) - r0);
+  auto refill = [&](int i) {        // thread 0: row r0 + i into its slot
+    uint64_t* bar = &full[i % p.stages];
+    uint8_t* slot = ring + (size_t)(i % p.stages) * tensors * row_bytes;
+    const int64_t off = (r0 + i) * cols;
+    mbar_expect_tx(bar, tensors * row_bytes);
+    bulk_copy(slot, x + off, row_bytes, bar);
+    bulk_copy(slot + row_bytes, dy + off, row_bytes, bar);
+    if (dres) bulk_copy(slot + 2 * (size_t)row_bytes, dres + off, row_bytes, bar);
+  };
+  if (threadIdx.x == 0) {
+    abort_word = 0;
+    for (int i = 0; i < p.stages; ++i) mbar_init(&full[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int i = 0; i < min(n, p.stages); ++i) refill(i);
+  }
+  // wide rows (VPT >= 4) are read from their slot a second time and w from the cache: held in registers, they would spill
+  constexpr bool HOLD = VPT < 4;
+  constexpr int NH = HOLD ? VPT : 1;
   float dwacc[VPT][V];
+  Vec16<T> wreg[NH], xb[NH], gb[NH], rb[NH];
+  auto load_w = [&](int c) {
+    const int i = threadIdx.x + c * THREADS;
 #pragma unroll
-  for (int c = 0; c < VPT; ++c)
+    for (int k = 0; k < V; ++k) wreg[HOLD ? c : 0].v[k] = ToF<T>::from(1.f);
+    if (w && i < nvec) wreg[HOLD ? c : 0] = ld16(w + (int64_t)i * V);
+  };
+#pragma unroll
+  for (int c = 0; c < VPT; ++c) {
 #pragma unroll
     for (int k = 0; k < V; ++k) dwacc[c][k] = 0.f;
-  Vec16<T> wreg[VPT];
-  {
-    int cnt;
-    _Pragma("unroll") for (cnt = 0; cnt < VPT; ++cnt) { const int i = threadIdx.x + cnt * THREADS; if (i >= nvec) break;
-      if (w) wreg[cnt] = ld16(w + (int64_t)i * V);
-      else {
+    if (HOLD) load_w(c);
+  }
+  __syncthreads();
+  float rs_next = n > 0 ? rstd[r0] : 0.f;
+  bool ok = true;
+  for (int r = 0; r < n; ++r) {
+    const float rs = rs_next;
+    if (r + 1 < n) rs_next = rstd[r0 + r + 1];
+    const uint8_t* slot = ring + (size_t)(r % p.stages) * tensors * row_bytes;
+    const T* sx = reinterpret_cast<const T*>(slot);
+    const T* sg = reinterpret_cast<const T*>(slot + row_bytes);
+    const T* sr = reinterpret_cast<const T*>(slot + 2 * (size_t)row_bytes);
+    const bool arrived = mbar_wait(&full[r % p.stages], (uint32_t)((r / p.stages) & 1), abort_flag);
+    auto load_row = [&](int c) {
+      const int i = threadIdx.x + c * THREADS, d = HOLD ? c : 0;
+      xb[d] = ld16(sx + (int64_t)i * V);
+      gb[d] = ld16(sg + (int64_t)i * V);
+      if (dres) rb[d] = ld16(sr + (int64_t)i * V);
+      if (!HOLD) load_w(c);
+    };
+    float dot = 0.f;
 #pragma unroll
-        for (int k = 0; k < V; ++k) wreg[cnt].v[k] = ToF<T>::from(1.f);
+    for (int c = 0; c < VPT; ++c) {
+      if (threadIdx.x + c * THREADS < nvec) {
+        const int d = HOLD ? c : 0;
+        load_row(c);
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          const float xh = ToF<T>::to(xb[d].v[k]) * rs;
+          const float g = ToF<T>::to(gb[d].v[k]);
+          dot += g * ToF<T>::to(wreg[d].v[k]) * xh;
+          dwacc[c][k] += g * xh;
+        }
       }
+    }
+    dot = warp_sum(dot);
+    if (lane == 0) sh[r & 1][wid] = dot;
+    ok = __syncthreads_and(arrived);
+    if (!ok) break;
+    if (HOLD && threadIdx.x == 0 && r + p.stages < n) refill(r + p.stages);
+    dot = warp_sum(lane < THREADS / 32 ? sh[r & 1][lane] : 0.f);
+    const float m = dot / (float)cols;
+#pragma unroll
+    for (int c = 0; c < VPT; ++c) {
+      const int i = threadIdx.x + c * THREADS;
+      if (i < nvec) {
+        const int d = HOLD ? c : 0;
+        if (!HOLD) load_row(c);
+        Vec16<T> o;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          const float xh = ToF<T>::to(xb[d].v[k]) * rs;
+          const float g = ToF<T>::to(gb[d].v[k]) * ToF<T>::to(wreg[d].v[k]);
+          float v = rs * (g - xh * m);
+          if (dres) v += ToF<T>::to(rb[d].v[k]);
+          o.v[k] = ToF<T>::from(v);
+        }
+        st16_stream(dx + (r0 + r) * cols + (int64_t)i * V, o);
+      }
+    }
+    if (!HOLD) {
+      __syncthreads();
+      if (threadIdx.x == 0 && r + p.stages < n) refill(r + p.stages);
     }
   }
-  const int64_t r0 = (int64_t)blockIdx.x * rows_per_cta;
-  const int64_t r1 = min(r0 + (int64_t)rows_per_cta, rows);
-  for (int64_t row = r0; row < r1; ++row) {
-    const T* xr = x + row * cols;
-    const T* gr = dy + row * cols;
-    const float rs = rstd[row];
-    Vec16<T> xb[VPT], gb[VPT];
-    float dot = 0.f;
-    int cnt;
-    _Pragma("unroll") for (cnt = 0; cnt < VPT; ++cnt) { const int i = threadIdx.x + cnt * THREADS; if (i >= nvec) break;
-      xb[cnt] = ld16_stream(xr + (int64_t)i * V);
-      gb[cnt] = ld16_stream(gr + (int64_t)i * V);
-#pragma unroll
-      for (int k = 0; k < V; ++k) {
-        float xh = ToF<T>::to(xb[cnt].v[k]) * rs;
-        float g = ToF<T>::to(gb[cnt].v[k]);
-        dot += g * ToF<T>::to(wreg[cnt].v[k]) * xh;
-        dwacc[cnt][k] += g * xh;
-      }
+  if (!ok) {       // the copies in flight get a bounded moment to land before the shared memory is released
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < 200; ++i) __nanosleep(1000);
+      if (p.status) atomicExch(p.status, 1);
     }
-    dot = block_sum(dot, sh);
-    const float m = dot / (float)cols;
-      _Pragma("unroll") for (cnt = 0; cnt < VPT; ++cnt) { const int i = threadIdx.x + cnt * THREADS; if (i >= nvec) break;
-      Vec16<T> o;
-#pragma unroll
-      for (int k = 0; k < V; ++k) {
-        float xh = ToF<T>::to(xb[cnt].v[k]) * rs;
-        float g = ToF<T>::to(gb[cnt].v[k]) * ToF<T>::to(wreg[cnt].v[k]);
-        o.v[k] = ToF<T>::from(rs * (g - xh * m));
-      }
-      st16_stream(dx + row * cols + (int64_t)i * V, o);
-    }
+    __syncthreads();
+    return;
   }
   if (dw_partial) {
     float* out = dw_partial + (int64_t)blockIdx.x * cols;
-    int cnt;
-    _Pragma("unroll") for (cnt = 0; cnt < VPT; ++cnt) { const int i = threadIdx.x + cnt * THREADS; if (i >= nvec) break;
 #pragma unroll
-      for (int k = 0; k < V; k += 4)
-        *reinterpret_cast<float4*>(out + (int64_t)i * V + k) =
-            make_float4(dwacc[cnt][k], dwacc[cnt][k + 1], dwacc[cnt][k + 2], dwacc[cnt][k + 3]);
+    for (int c = 0; c < VPT; ++c) {
+      const int i = threadIdx.x + c * THREADS;
+      if (i < nvec) {
+#pragma unroll
+        for (int k = 0; k < V; k += 4)
+          *reinterpret_cast<float4*>(out + (int64_t)i * V + k) =
+              make_float4(dwacc[c][k], dwacc[c][k + 1], dwacc[c][k + 2], dwacc[c][k + 3]);
+      }
     }
   }
 }
@@ -254,6 +347,33 @@ __global__ void __launch_bounds__(THREADS) layernorm_bwd_kernel(T* __restrict__ 
 
 constexpr int64_t kMaxRowVecs = 512 * 8;
 
+// Two CTAs per SM walk strips of rows; each gets half of the shared memory for its ring, or, where a row is so wide that
+// not even two slots fit into that half, all of it (one CTA per SM at a time then).  Four slots of 24 KB (4096 bf16 columns
+// with dres) already keep 190 KB per SM in flight; more are not used.
+template <typename T, int THREADS, int VPT>
+int rmsnorm_bwd_go(int nb, cudaStream_t stream, T* dx, float* dwp, const T* dy, const T* x, const T* w, const float* rstd, const T* dres,
+                   RmsBwdParams p) {
+  constexpr int kHalf = 112 * 1024, kWhole = 224 * 1024;
+  const int64_t slot = p.cols * (int64_t)sizeof(T) * (dres ? 3 : 2);
+  const int64_t room = slot * 2 <= kHalf ? kHalf : kWhole;
+  p.stages = (int)std::min<int64_t>(room / slot, kMaxRmsStages);
+  if (p.stages < 1) return (int)cudaErrorNotSupported;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(rmsnorm_bwd_kernel<T, THREADS, VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWhole);
+  if (attr != cudaSuccess) return (int)attr;
+  rmsnorm_bwd_kernel<T, THREADS, VPT><<<nb, THREADS, p.stages * slot, stream>>>(dx, dwp, dy, x, w, rstd, dres, p);
+  B200K_LAUNCH_RET();
+}
+template <typename T, typename... A>
+int rmsnorm_bwd_launch(int64_t nvec, A... args) {
+  if (nvec <= 128) return rmsnorm_bwd_go<T, 128, 1>(args...);
+  if (nvec <= 256) return rmsnorm_bwd_go<T, 256, 1>(args...);
+  if (nvec <= 512) return rmsnorm_bwd_go<T, 256, 2>(args...);
+  if (nvec <= 1024) return rmsnorm_bwd_go<T, 512, 2>(args...);
+  if (nvec <= 2048) return rmsnorm_bwd_go<T, 512, 4>(args...);
+  return rmsnorm_bwd_go<T, 512, 8>(args...);
+}
+
 }  // namespace
 }  // namespace b200k
 
@@ -287,7 +407,7 @@ int b200_rmsnorm_fwd(int dtype, void* y, float* rstd, const void* x, const void*
 }
 
 int b200_rmsnorm_bwd(int dtype, void* dx, float* dw_partial, int* nblocks_out_host, const void* dy, const void* x,
-                     const void* w, const float* rstd, int64_t rows, int64_t cols, cudaStream_t stream) {
+                     const void* w, const float* rstd, const void* dres, int64_t rows, int64_t cols, cudaStream_t stream) {
   if (rows == 0) return 0;
   int nb = b200_rmsnorm_bwd_partial_rows(rows, cols);
   int rpc = (int)cdiv(rows, nb);
@@ -296,11 +416,10 @@ int b200_rmsnorm_bwd(int dtype, void* dx, float* dw_partial, int* nblocks_out_ho
     constexpr int V = Vec16<T>::N;
     int64_t nvec = cols / V;
     if (cols % V != 0 || nvec > kMaxRowVecs || !aligned16((const T*)x) || !aligned16((const T*)dy) ||
-        !aligned16((T*)dx) || (w && !aligned16((const T*)w)))
+        !aligned16((T*)dx) || (w && !aligned16((const T*)w)) || (dres && !aligned16((const T*)dres)))
       return (int)cudaErrorNotSupported;
-    B200K_ROW_LAUNCH(rmsnorm_bwd_kernel, nvec, nb, stream, (T*)dx, dw_partial, (const T*)dy, (const T*)x, (const T*)w,
-                     rstd, rows, cols, rpc);
-    B200K_LAUNCH_RET();
+    RmsBwdParams p{rows, cols, rpc, 0, gemm_status_word_device()};
+    return rmsnorm_bwd_launch<T>(nvec, nb, stream, (T*)dx, dw_partial, (const T*)dy, (const T*)x, (const T*)w, rstd, (const T*)dres, p);
   })
   return (int)cudaErrorNotSupported;
 }

@@ -23,7 +23,7 @@ def register() -> None:
         return
     _registered = True
     try:
-        from torch.distributed.tensor import Replicate, Shard
+        from torch.distributed.tensor import Partial, Replicate, Shard
         from torch.distributed.tensor.experimental import register_sharding
     except Exception:  # pragma: no cover  (torch built without distributed)
         return
@@ -74,6 +74,19 @@ def register() -> None:
             # outputs: normalised, new residual (shaped like x) and the per-row rstd (one dimension fewer)
             rules.append(([Shard(d), Shard(d), Shard(d)], [Shard(d), Shard(d), Replicate()]))
         return rules
+
+    @register_sharding(ops.rms_norm_residual_backward.default)
+    def _rms_norm_residual_backward(dy, dres, res, rstd, weight):
+        n = 4 + (dres is not None)
+        rules = [([Replicate()] * 2, [Replicate()] * n)]
+        for d in range(res.ndim - 1):
+            # rows are independent; every shard adds its part of the weight's gradient
+            rules.append(([Shard(d), Partial()], [Shard(d)] * (n - 1) + [Replicate()]))
+        return rules
+
+    @register_sharding(ops.cross_entropy_mean.default)
+    def _ce_mean(loss_rows, target, ignore_index=-100):
+        return [([Replicate(), Replicate()], [Replicate(), Replicate()])]     # a mean over all rows
 
     @register_sharding(ops.cross_entropy_fwd.default)
     def _ce_fwd(logits, target, ignore_index=-100, label_smoothing=0.0):

@@ -70,6 +70,16 @@ def _(x, residual, weight, eps):
     return torch.empty_like(x), torch.empty_like(x), stat
 
 
+@_reg("rms_norm_residual_backward")
+def _(dy, dres, res, rstd, weight):
+    return torch.empty_like(res, memory_format=torch.contiguous_format), torch.empty_like(weight, memory_format=torch.contiguous_format)
+
+
+@_reg("cross_entropy_mean")
+def _(loss_rows, target, ignore_index=-100):
+    return loss_rows.new_empty(()), loss_rows.new_empty(())
+
+
 @_reg("multi_tensor_l2norm")
 def _(tensors, per_tensor=False):
     t = tensors[0]

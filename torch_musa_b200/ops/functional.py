@@ -30,10 +30,7 @@ class _RMSNormResidual(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dres):
         res, weight, rstd = ctx.saved_tensors
-        dx, dw = torch.ops.aten._fused_rms_norm_backward(dy.contiguous(), res, [res.shape[-1]], rstd, weight,
-                                                         [True, True])
-        if dres is not None:
-            dx = dx + dres
+        dx, dw = torch.ops.blackwell.rms_norm_residual_backward(dy, dres, res, rstd, weight)
         return dx, dx, dw, None
 
 
@@ -297,8 +294,7 @@ class _FusedCE(torch.autograd.Function):
         loss_rows, lse = torch.ops.blackwell.cross_entropy_fwd(logits, target, ignore_index, label_smoothing)
         n_valid = None
         if reduction == "mean":
-            n_valid = (target != ignore_index).sum().clamp_min(1).to(torch.float32)
-            out = loss_rows.sum() / n_valid
+            out, n_valid = torch.ops.blackwell.cross_entropy_mean(loss_rows, target, ignore_index)
         elif reduction == "sum":
             out = loss_rows.sum()
         else:
