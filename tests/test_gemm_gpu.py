@@ -228,3 +228,34 @@ def test_grouped_gemm_device_side_counts(bw, dev, counts, R):
     # the host implementation of the same contract (any device) agrees
     y_cpu = grouped_linear(x.float(), w.float(), cnt)
     assert torch.allclose(y_cpu[:used], y_ref[:used], atol=1e-4)
+
+
+@pytest.mark.parametrize("m", [1, 15, 17, 33, 64])
+@pytest.mark.parametrize("n,k", [(64, 256), (1000, 328), (4096, 4096), (129, 2048), (20008, 264), (24, 512)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_few_rows(bw, dev, m, n, k, dt):
+    """The few-row kernel at the edges of its row paddings, with remainders of N (also ones that rule out vector stores) and K,
+    one CTA and clusters of up to eight per tile; bias, activation and accumulation in its epilogue.  24 columns take the
+    general kernel."""
+    torch.manual_seed(m + n)
+    x, w, b, c = torch.randn(m, k).to(dt), (torch.randn(n, k) * 0.1).to(dt), torch.randn(n).to(dt), torch.randn(m, n).to(dt)
+    xd, wd, bd, cd = (t.to(dev) for t in (x, w, b, c))
+    ref = x.double() @ w.double().t()
+    eps = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+
+    def check(got, want):
+        # fp32 sums of k products, then one rounding to the type (two with a rounded addend)
+        lim = 2 * eps * want.abs() + 1e-6 * k
+        assert ((got.double().cpu() - want).abs() <= lim).all()
+
+    first = torch.nn.functional.linear(xd, wd)
+    check(first, ref)
+    assert torch.equal(first, torch.nn.functional.linear(xd, wd))        # the order of the sums does not depend on timing
+    check(torch.nn.functional.linear(xd, wd, bd), ref + b.double())
+    check(torch.ops.aten._addmm_activation(bd, xd, wd.t()), (ref + b.double()).relu())
+    check(torch.addmm(cd, xd, wd.t(), beta=1.0, alpha=0.5), c.double() + 0.5 * ref)
+    wide = torch.empty(m, n + 3, dtype=dt, device=dev)[:, 1:n + 1]       # rows that start off any vector boundary
+    torch.mm(xd, wd.t(), out=wide)
+    check(wide, ref)
+    bw.synchronize()
+    assert bw._C._gemm_status(False) == 0

@@ -138,6 +138,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor (sm_100 format): 128-byte swizzle, version 1.
@@ -288,6 +297,7 @@ struct RsParams {
 
 // What the host decided for one problem: how many K-splits and which kernel family.
 struct GemmPlan {
+  int skinny;        // 1: few-row kernel (gemm_skinny.cu)
   int pair;          // 1: SM-pair kernel (256-row tiles), 0: single-CTA kernel (128-row tiles)
   int dynamic;       // pair kernel: cluster-launch-control schedule
   int splits;        // 1 = no split-K
@@ -303,6 +313,9 @@ int gemm_sm_count();
 int gemm_launch_2cta(const b200_gemm_desc_t* g, void* d, const void* a, const void* b, cudaStream_t stream,
                      const GemmPlan& plan, const AgParams* ag = nullptr, const RsParams* rs = nullptr);
 GemmPlan gemm_plan(const b200_gemm_desc_t* g);
+// few rows: whether the kernel of gemm_skinny.cu is the better one, and its launch
+bool gemm_skinny_fits(const b200_gemm_desc_t* g);
+int gemm_launch_skinny(const b200_gemm_desc_t* g, void* d, const void* a, const void* b, cudaStream_t stream);
 // sums the fp32 partial products of a split-K run and applies bias / activation / accumulate / output cast
 int gemm_splitk_reduce(const b200_gemm_desc_t* g, void* d, const float* ws, int splits, cudaStream_t stream);
 

@@ -493,6 +493,7 @@ static int gemm_validate(const b200_gemm_desc_t* g, const void* a, const void* b
 
 static int gemm_dispatch(const b200_gemm_desc_t* g, void* d, const void* a, const void* b, cudaStream_t stream,
                          const GemmPlan& plan) {
+  if (plan.skinny) return gemm_launch_skinny(g, d, a, b, stream);
   if (plan.pair) return gemm_launch_2cta(g, d, a, b, stream, plan);
   switch (g->out_dtype) {
     case B200_BF16: return launch<__nv_bfloat16>(g, d, a, b, stream, plan);

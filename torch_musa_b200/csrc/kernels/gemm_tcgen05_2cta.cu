@@ -774,6 +774,13 @@ GemmPlan gemm_plan(const b200_gemm_desc_t* g) {
     }
   }
   GemmPlan plan;
+  plan.skinny = forced == 0 && gemm_skinny_fits(g);
+  if (plan.skinny) {
+    plan.pair = plan.dynamic = 0;
+    plan.splits = 1;          // it splits K inside clusters, without a workspace
+    plan.kb_per_split = (g->k + BK - 1) / BK;
+    return plan;
+  }
   plan.pair = choice == 2 || choice == 3;
   plan.dynamic = choice == 3;
   const bool tf32 = g->in_dtype == B200_F32;  // fp32 operands: single-CTA kernel, 32 elements per K block, no split
@@ -898,6 +905,7 @@ extern "C" int b200_gemm_allgather(const b200_gemm_desc_t* g, const b200_symm_t*
   ag.epoch = epoch;
   if (int e = sync_wait_limit(ag.wait_cycles, stream)) return e;
   GemmPlan plan;
+  plan.skinny = 0;
   plan.pair = 1;
   plan.dynamic = 0;
   plan.splits = 1;
@@ -935,6 +943,7 @@ extern "C" int b200_gemm_reduce_scatter(const b200_gemm_desc_t* g, const b200_sy
   rs.epoch = epoch;
   if (int e = sync_wait_limit(rs.wait_cycles, stream)) return e;
   GemmPlan plan;
+  plan.skinny = 0;
   plan.pair = 1;
   plan.dynamic = 0;
   plan.splits = 1;
