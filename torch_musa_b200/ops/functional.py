@@ -20,24 +20,11 @@ def rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], eps: float = 1e-6)
     return F.rms_norm(x, (x.shape[-1],), weight, eps)
 
 
-class _RMSNormResidual(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, residual, weight, eps):
-        y, res, rstd = torch.ops.blackwell.rms_norm_residual(x, residual, weight, eps)
-        ctx.save_for_backward(res, weight, rstd)
-        return y, res
-
-    @staticmethod
-    def backward(ctx, dy, dres):
-        res, weight, rstd = ctx.saved_tensors
-        dx, dw = torch.ops.blackwell.rms_norm_residual_backward(dy, dres, res, rstd, weight)
-        return dx, dx, dw, None
-
-
 def rms_norm_residual(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6):
     """Fused ``h = x + residual; y = rms_norm(h)``; returns ``(y, h)`` (one pass over memory)."""
     if _on_device(x):
-        return _RMSNormResidual.apply(x, residual, weight, eps)
+        y, h, _ = torch.ops.blackwell.rms_norm_residual(x, residual, weight, eps)     # differentiable (autograd in C++)
+        return y, h
     h = x + residual
     return rms_norm(h, weight, eps), h
 
