@@ -262,8 +262,9 @@ std::tuple<at::Tensor, at::Tensor> rms_norm_residual_backward(const at::Tensor& 
 }
 
 // Autograd of rms_norm_residual in C++: the operation is called once per sub-layer on rows that take a few microseconds, and
-// the interpreter's part of a Python autograd function was most of a call (32 x 4096 rows without gradients: 13.3 us a call
-// before, HOST_FWD now; 4096 x 4096 with both directions: 95 us against 55 us of kernels before, HOST_TRAIN now).
+// the interpreter's part of a Python autograd function was most
+// of a call (32 x 4096 rows without gradients: 13.1 us a call
+// before, 8.4 now; 4096 x 4096 with both directions: 95 us against 55 us of kernels before, 87 now).
 using RmsResidualOut = std::tuple<at::Tensor, at::Tensor, at::Tensor>;
 RmsResidualOut call_rms_norm_residual(const at::Tensor& x, const at::Tensor& residual, const at::Tensor& weight, double eps) {
   static auto op = c10::Dispatcher::singleton()

@@ -130,9 +130,10 @@ class LlamaDecoder:
     def _step(self) -> None:
         m, cfg, B = self.model, self.cfg, self.B
         hd, h, kv = cfg.head_dim, cfg.n_heads // self.tp, cfg.kv_heads // self.tp
-        positions = self.pos.expand(B, 1)
-        # keys at index <= pos are visible (additive mask, broadcast over batch and heads)
-        mask = torch.where(self._arange <= self.pos, 0.0, float("-inf")).to(self.k_cache.dtype).view(1, 1, 1, self.max_len)
+        if not self._fused_decode:     # (the fused kernels read the position themselves: four launches less per step)
+            positions = self.pos.expand(B, 1)
+            # keys at index <= pos are visible (additive mask, broadcast over batch and heads)
+            mask = torch.where(self._arange <= self.pos, 0.0, float("-inf")).to(self.k_cache.dtype).view(1, 1, 1, self.max_len)
         x = m.tok_emb(self.tokens)
         delta = None          # the previous block's output, added to the residual stream inside the next norm kernel
         for li, layer in enumerate(m.layers):
