@@ -74,3 +74,43 @@ def test_quantize_1x128(bw, dev):
     y = torch.ops.blackwell.scaled_mm(q, qw.to(dev), s, sw.to(dev), None, None, None, torch.bfloat16)
     ref = x.float() @ w.t()
     assert ((y.float().cpu() - ref).abs().max() / ref.abs().max()) < 0.08
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 128, 128), (129, 392, 384), (300, 5000, 256), (2600, 2056, 128), (1029, 4104, 1152)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_scaled_mm_tiles(bw, dev, m, n, k, out_dtype):
+    """Both tile widths, several tiles per CTA, remainders of rows, columns (also no multiple of a vector store) and an odd
+    number of K blocks, with every factor and the bias of the epilogue."""
+    torch.manual_seed(m)
+    qa, sa = quant_blocks(torch.randn(m, k), 1)
+    npad = (n + 127) // 128 * 128
+    bpad = torch.zeros(npad, k)
+    bpad[:n] = torch.randn(n, k) * 0.5
+    qb_p, sb = quant_blocks(bpad, 128)
+    qb = qb_p[:n].contiguous()
+    ra, rb, bias = torch.rand(m) + 0.5, torch.rand(n) + 0.5, torch.randn(n)
+    want = (dequant(qa, sa, 1).double() @ dequant(qb_p, sb, 128)[:n].double().t()) * ra.double()[:, None] * rb.double() + bias.double()
+    y = torch.ops.blackwell.scaled_mm(qa.to(dev), qb.to(dev), sa.to(dev), sb.to(dev), ra.to(dev), rb.to(dev), bias.to(dev), out_dtype)
+    # a block product keeps its leading bits only as far as the fp8 tensor core does (2^-13 of its largest term); the rounding of
+    # the output comes on top
+    lim = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -11
+    assert float((y.double().cpu() - want).abs().max()) <= lim * float(want.abs().max())
+    bw.synchronize()
+    assert bw._C._gemm_status(False) == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,k", [(1, 128), (5, 1152), (67, 4096)])
+def test_quantize_routes_agree(bw, dev, dt, rows, k):
+    """The vectorised quantiser and the one for any alignment give the same bytes and scales."""
+    torch.manual_seed(rows)
+    x = (torch.randn(rows, k) * 3).to(dt)
+    x[0, :128] = 0
+    xd = x.to(dev)
+    # a leading dimension of k + 4: with 16-bit elements no row but the first starts on 16 bytes; with 32-bit ones the base does not
+    off = torch.empty(rows * (k + 4) + 1, dtype=dt, device=dev)[(1 if dt == torch.float32 else 0):].as_strided((rows, k), (k + 4, 1))
+    off.copy_(xd)
+    for e5m2 in (False, True):
+        q0, s0 = torch.ops.blackwell.quantize_fp8_1x128(xd, e5m2)
+        q1, s1 = torch.ops.blackwell.quantize_fp8_1x128(off, e5m2)
+        assert torch.equal(q0.cpu().view(torch.uint8), q1.cpu().view(torch.uint8)) and torch.equal(s0.cpu(), s1.cpu())
