@@ -433,3 +433,41 @@ def test_fused_cross_entropy_row_widths(bw, dev, rows, cols, dt):
     assert float((xd.grad.double().cpu() - xr.grad).abs().max()) <= lim * float(xr.grad.abs().max())
     none = fused_cross_entropy(x.to(dev), torch.full((rows,), -100).to(dev))
     assert float(none) == 0.0
+
+
+# One aligned 16-byte group, a whole half, and all of the row at a finite mask value; logits far from zero.
+@pytest.mark.parametrize("rows,cols", [(6, 1024), (6, 4096), (6, 32000), (1300, 1024), (700, 4104)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_row_statistics_masked_and_offset(bw, dev, dt, rows, cols):
+    from torch_musa_b200.ops import fused_cross_entropy
+
+    torch.manual_seed(rows + cols)
+    base = torch.randn(rows, cols, dtype=torch.float64) * 3
+    cases = [("offset", base + 1e3), ("offset", base + 1e5)]
+    for value in (torch.finfo(dt).min, -1e9, -1e10, -1e30):
+        for part in (slice(8, 16), slice(0, cols // 2), slice(0, cols)):
+            x = base.clone()
+            x[:, part] = value
+            cases.append(("mask", x))
+    t = torch.randint(cols // 2, cols, (rows,))
+    for kind, x in cases:
+        x = x.to(dt)
+        d, xd = x.double(), x.to(dev)
+        m = d.amax(-1, keepdim=True)
+        # in the exponent, x - m and its product with log2(e) are each rounded once to 24 bits; the terms that count are
+        # within 30 of the maximum; 2^x and the four-way sums add a few units in the last place
+        rel = 30 * 2.0 ** -23 + 8 * 2.0 ** -22
+        out = 2.0 ** -8 if dt is torch.bfloat16 else 2.0 ** -23
+        p = torch.softmax(d, -1)
+        got = torch.softmax(xd, -1).cpu().double()
+        assert torch.allclose(got, p, rtol=rel + out, atol=1e-13), (kind, float((got - p).abs().max()))
+        stats = torch.ops.blackwell.online_softmax_stats(xd, t.to(dev), 0).cpu().double()
+        assert torch.equal(stats[:, 0], m[:, 0])
+        assert torch.allclose(stats[:, 1], (d - m).exp().sum(-1), rtol=rel, atol=0.0)
+        # the log-sum-exp itself has to fit into 24 bits
+        atol = float(m.abs().max()) * 2.0 ** -23 + 2e-5
+        logp = torch.log_softmax(d, -1)
+        got = torch.log_softmax(xd, -1).cpu().double()
+        assert torch.allclose(got, logp, rtol=out, atol=atol), (kind, float((got - logp).abs().max()))
+        loss = fused_cross_entropy(xd, t.to(dev), reduction="none").cpu().double()
+        assert torch.allclose(loss, F.cross_entropy(d, t, reduction="none"), rtol=2.0 ** -22, atol=atol)

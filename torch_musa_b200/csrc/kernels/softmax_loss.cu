@@ -55,50 +55,56 @@ __device__ __forceinline__ float exp2f_approx(float x) {
   return y;
 }
 
+// N vectors of a row into the running (maximum, sum): the maximum in four chains, one correction of the sum, then the
+// exponentials in four chains of additions.  The maximum is subtracted before the scaling by log2(e): rounded on its own,
+// the product m * log2(e) would put its error, or for masks near the type's lowest value its overflow, into every term.
+template <int N, typename T>
+__device__ __forceinline__ void ms_push_vecs(MaxSum& acc, const Vec16<T> (&v)[N]) {
+  constexpr int V = Vec16<T>::N;
+  constexpr float kLog2e = 1.4426950408889634f;
+  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+#pragma unroll
+    for (int k = 0; k < V; ++k) mx[k & 3] = fmaxf(mx[k & 3], ToF<T>::to(v[u].v[k]));
+  const float lm = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+  if (lm > acc.m) { acc.s *= __expf(acc.m - lm); acc.m = lm; }
+  if (acc.m == -INFINITY) return;
+  float sm[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+#pragma unroll
+    for (int k = 0; k < V; ++k) sm[k & 3] += exp2f_approx((ToF<T>::to(v[u].v[k]) - acc.m) * kLog2e);
+  acc.s += (sm[0] + sm[1]) + (sm[2] + sm[3]);
+}
+
 // Row statistics with optional 16-byte vector loads (VEC requires cols % V == 0 and an aligned base).
 template <typename T, bool VEC>
 __device__ __forceinline__ MaxSum row_stats(const T* __restrict__ xr, int64_t cols, float* shm, float* shs) {
   constexpr int V = Vec16<T>::N;
   MaxSum acc{-INFINITY, 0.f};
   if constexpr (VEC) {
-    // Four 16-byte loads per thread are in flight while the four before them are worked on: the maximum in four chains, one
-    // correction of the running sum, then the exponentials as 2^(x log2(e) - m log2(e)) in four chains of additions.
+    // Four 16-byte loads per thread are in flight while the four before them are worked on.
     const int nvec = (int)(cols / V), step = blockDim.x * 4;
-    constexpr float kLog2e = 1.4426950408889634f;
     Vec16<T> cur[4], nxt[4];
     auto load = [&](Vec16<T>(&v)[4], int i0) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int i = i0 + u * blockDim.x;
         if (i < nvec) v[u] = ld16(xr + (int64_t)i * V);
-        else {
-#pragma unroll
-          for (int k = 0; k < V; ++k) v[u].v[k] = ToF<T>::from(-INFINITY);
-        }
       }
     };
     load(cur, threadIdx.x);
-    for (int i0 = threadIdx.x; i0 < nvec; i0 += step) {
+    int i0 = threadIdx.x;
+    for (; i0 - (int)threadIdx.x + step <= nvec; i0 += step) {     // whole groups: every thread has four vectors
       load(nxt, i0 + step);
-      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int k = 0; k < V; ++k) mx[k & 3] = fmaxf(mx[k & 3], ToF<T>::to(cur[u].v[k]));
-      const float lm = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      if (lm > acc.m) { acc.s *= __expf(acc.m - lm); acc.m = lm; }
-      if (acc.m != -INFINITY) {
-        const float neg = -acc.m * kLog2e;
-        float sm[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int k = 0; k < V; ++k) sm[k & 3] += exp2f_approx(fmaf(ToF<T>::to(cur[u].v[k]), kLog2e, neg));
-        acc.s += (sm[0] + sm[1]) + (sm[2] + sm[3]);
-      }
+      ms_push_vecs<4>(acc, cur);
 #pragma unroll
       for (int u = 0; u < 4; ++u) cur[u] = nxt[u];
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * (int)blockDim.x < nvec) ms_push_vecs<1>(acc, reinterpret_cast<const Vec16<T>(&)[1]>(cur[u]));
   } else {
     for (int64_t i = threadIdx.x; i < cols; i += blockDim.x) ms_push(acc, ToF<T>::to(xr[i]));
   }
