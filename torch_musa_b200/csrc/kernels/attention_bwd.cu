@@ -546,7 +546,7 @@ int bwd_setup(K kern) {
   cudaError_t e = cudaFuncGetAttributes(&at, kern);
   if (e != cudaSuccess) return (int)e;
   if (at.numRegs < kLaunchRegs) return (int)cudaErrorNotSupported;   // the register split would wait for ever
-  return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
+  return opt_in_smem(kern, kBwdSmem);
 }
 
 }  // namespace
@@ -615,15 +615,15 @@ extern "C" int b200_flash_attn_bwd(const b200_attn_t* a, float* dq_accum, void* 
   const int row_blocks = (dS + kDeltaRows - 1) / kDeltaRows;
   const unsigned delta_grid = (unsigned)((long long)dB * a->H * row_blocks);
   if (bf16) {
-    static const int setup = bwd_setup(attn_bwd_kernel<__nv_bfloat16>);
-    if (setup != 0) return setup;
+    static OncePerDevice once;
+    if (int e = once([] { return bwd_setup(attn_bwd_kernel<__nv_bfloat16>); })) return e;
     attn_delta_kernel<__nv_bfloat16><<<delta_grid, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, dq_accum,
                                                                      a->H, dS, row_blocks, a->o_sb, a->o_sh, a->o_ss, x[0], x[1], x[2]);
     attn_bwd_kernel<__nv_bfloat16><<<(unsigned)grid, kBwdThreads, kBwdSmem, stream>>>(mq, mk, mv, mdo, mdq, (__nv_bfloat16*)dk,
                                                                                      (__nv_bfloat16*)dv, p);
   } else {
-    static const int setup = bwd_setup(attn_bwd_kernel<__half>);
-    if (setup != 0) return setup;
+    static OncePerDevice once;
+    if (int e = once([] { return bwd_setup(attn_bwd_kernel<__half>); })) return e;
     attn_delta_kernel<__half><<<delta_grid, 256, 0, stream>>>((const __half*)o, (const __half*)d_o, delta, dq_accum, a->H, dS, row_blocks,
                                                               a->o_sb, a->o_sh, a->o_ss, x[0], x[1], x[2]);
     attn_bwd_kernel<__half><<<(unsigned)grid, kBwdThreads, kBwdSmem, stream>>>(mq, mk, mv, mdo, mdq, (__half*)dk, (__half*)dv, p);

@@ -379,7 +379,7 @@ int fwd_setup(K kern) {
   cudaError_t e = cudaFuncGetAttributes(&at, kern);
   if (e != cudaSuccess) return (int)e;
   if (at.numRegs < kLaunchRegs) return (int)cudaErrorNotSupported;   // the register split would wait for ever
-  return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
+  return opt_in_smem(kern, kAttnSmem);
 }
 
 }  // namespace
@@ -432,12 +432,12 @@ extern "C" int b200_flash_attn_fwd(const b200_attn_t* a, void* out, float* lse, 
   const long long grid = (long long)a->B * a->H * p.q_pairs;
   if (grid > 2147483647ll) return (int)cudaErrorNotSupported;
   if (bf16) {
-    static const int e = fwd_setup(attn_fwd_kernel<__nv_bfloat16>);
-    if (e != 0) return e;
+    static OncePerDevice once;
+    if (int e = once([] { return fwd_setup(attn_fwd_kernel<__nv_bfloat16>); })) return e;
     attn_fwd_kernel<__nv_bfloat16><<<(unsigned)grid, kAttnThreads, kAttnSmem, stream>>>(mq, mk, mv, (__nv_bfloat16*)out, p);
   } else {
-    static const int e = fwd_setup(attn_fwd_kernel<__half>);
-    if (e != 0) return e;
+    static OncePerDevice once;
+    if (int e = once([] { return fwd_setup(attn_fwd_kernel<__half>); })) return e;
     attn_fwd_kernel<__half><<<(unsigned)grid, kAttnThreads, kAttnSmem, stream>>>(mq, mk, mv, (__half*)out, p);
   }
   B200K_LAUNCH_RET();

@@ -104,6 +104,28 @@ __device__ __forceinline__ float block_max(float v, float* sh) {
   return r;
 }
 
+// Set-up of a kernel that is made once: the opt-in to more than 48 KB of dynamic shared memory, and the checks beside it.  A
+// function's attributes belong to one device's copy of it, so the result is remembered per device.
+struct OncePerDevice {
+  static constexpr int kDevices = 64;
+  std::atomic<int> result[kDevices];      // 0: not yet; otherwise the error code + 1
+  template <typename F>
+  int operator()(F setup) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev >= kDevices) return setup();
+    if (int r = result[dev].load(std::memory_order_acquire)) return r - 1;
+    const int r = setup();
+    result[dev].store(r + 1, std::memory_order_release);
+    return r;
+  }
+};
+template <typename K>
+inline int opt_in_smem(K kernel, int bytes) {
+  return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 template <typename T>

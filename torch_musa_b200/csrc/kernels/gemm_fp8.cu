@@ -307,13 +307,14 @@ int launch_fp8(const b200_fp8_gemm_t* g, void* d, const void* a, const void* b, 
   p.group_m = gemm_group_m(FM, g->m, g->k / 2);     // one byte per element
   using C = F8Cfg<FN>;
   auto kern = gemm_fp8_kernel<OutT, FN>;
-  static const int setup = [&] {
+  static OncePerDevice once;
+  const int setup = once([&] {
     cudaFuncAttributes at;
     cudaError_t e = cudaFuncGetAttributes(&at, kern);
     if (e != cudaSuccess) return (int)e;
     if (at.numRegs < kLaunchRegs) return (int)cudaErrorNotSupported;   // the register split would wait for ever
-    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
-  }();
+    return opt_in_smem(kern, C::kSmem);
+  });
   if (setup != 0) return setup;
   const int grid = std::min(p.tiles_m * p.tiles_n, gemm_sm_count());
   kern<<<grid, kF8Threads, C::kSmem, stream>>>(ma, mb, (OutT*)d, p);

@@ -267,13 +267,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
 template <typename OutT, bool RAGGED_K, bool B_KMAJOR>
 int go(const CUtensorMap& ma, const CUtensorMap& mb, void* d, const GParams& p, int grid, cudaStream_t stream) {
-  static bool attr_set = false;
+  static OncePerDevice once;
   auto kern = grouped_gemm_kernel<OutT, RAGGED_K, B_KMAJOR>;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  if (int e = once([&] { return opt_in_smem(kern, kSmemBytes); })) return e;
   kern<<<grid, kThreads, kSmemBytes, stream>>>(ma, mb, (OutT*)d, p);
   B200K_LAUNCH_RET();
 }

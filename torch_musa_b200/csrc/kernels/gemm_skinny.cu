@@ -234,8 +234,8 @@ int go(const b200_gemm_desc_t* g, void* d, const void* a, const void* b, int spl
   p.status = gemm_status_word_device();
   p.splits = splits;
   auto kern = gemm_skinny_kernel<OutT, MP>;
-  static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
-  if (attr != cudaSuccess) return (int)attr;
+  static OncePerDevice once;
+  if (int e = once([&] { return opt_in_smem(kern, C::kSmem); })) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(((g->n + BN - 1) / BN) * splits));
   cfg.blockDim = dim3(kThreads);

@@ -400,25 +400,17 @@ int launch(const b200_gemm_desc_t* g, void* d, const void* a, const void* b, cud
 
 #define GEMM_GO(AK, BKM)                                                                                         \
   do {                                                                                                           \
-    static bool attr_set = false;                                                                                \
+    static OncePerDevice once;                                                                                   \
     auto kern = gemm_kernel<OutT, AK, BKM>;                                                                      \
-    if (!attr_set) {                                                                                             \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);       \
-      if (e != cudaSuccess) return (int)e;                                                                       \
-      attr_set = true;                                                                                           \
-    }                                                                                                            \
+    if (int e = once([&] { return opt_in_smem(kern, kSmemBytes); })) return e;                                   \
     kern<<<grid, kThreads, kSmemBytes, stream>>>(ma, mb, (OutT*)d, p);                                           \
   } while (0)
 
   if (tf32) {
     if constexpr (std::is_same<OutT, float>::value) {
-      static bool attr_set = false;
+      static OncePerDevice once;
       auto kern = gemm_kernel<float, true, true, true>;
-      if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        if (e != cudaSuccess) return (int)e;
-        attr_set = true;
-      }
+      if (int e = once([&] { return opt_in_smem(kern, kSmemBytes); })) return e;
       kern<<<grid, kThreads, kSmemBytes, stream>>>(ma, mb, (float*)d, p);
       B200K_LAUNCH_RET();
     } else {

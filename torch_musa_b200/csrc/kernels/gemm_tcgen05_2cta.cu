@@ -708,13 +708,9 @@ int launch_pair(const b200_gemm_desc_t* g, void* d, const void* a, const void* b
 
 #define GEMM2_GO(AK, BKM)                                                                                        \
   do {                                                                                                           \
-    static bool attr_set = false;                                                                                \
+    static OncePerDevice once;                                                                                   \
     auto kern = gemm_pair_kernel<OutT, AK, BKM, BN>;                                                             \
-    if (!attr_set) {                                                                                             \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);         \
-      if (e != cudaSuccess) return (int)e;                                                                       \
-      attr_set = true;                                                                                           \
-    }                                                                                                            \
+    if (int e = once([&] { return opt_in_smem(kern, C::kSmem); })) return e;                                     \
     kern<<<grid, kThreads, C::kSmem, stream>>>(ma, mb, (OutT*)d, p, dynamic, ag, rs);                                            \
   } while (0)
 

@@ -358,9 +358,8 @@ int rmsnorm_bwd_go(int nb, cudaStream_t stream, T* dx, float* dwp, const T* dy, 
   const int64_t room = slot * 2 <= kHalf ? kHalf : kWhole;
   p.stages = (int)std::min<int64_t>(room / slot, kMaxRmsStages);
   if (p.stages < 1) return (int)cudaErrorNotSupported;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(rmsnorm_bwd_kernel<T, THREADS, VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWhole);
-  if (attr != cudaSuccess) return (int)attr;
+  static OncePerDevice once;
+  if (int e = once([&] { return opt_in_smem(rmsnorm_bwd_kernel<T, THREADS, VPT>, kWhole); })) return e;
   rmsnorm_bwd_kernel<T, THREADS, VPT><<<nb, THREADS, p.stages * slot, stream>>>(dx, dwp, dy, x, w, rstd, dres, p);
   B200K_LAUNCH_RET();
 }
