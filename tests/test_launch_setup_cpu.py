@@ -21,9 +21,10 @@ DRIVER = r"""
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <string>
 #include <utility>
 
-static int g_dev = 0, g_launched = 0;
+static int g_dev = 0, g_fail = 0, g_launched = 0;
 static cudaError_t g_last = cudaSuccess;
 static std::map<std::pair<int, const void*>, size_t> g_opt_in;
 
@@ -47,6 +48,7 @@ cudaError_t cudaDeviceGetAttribute(int* v, enum cudaDeviceAttr, int) { *v = 148;
 cudaError_t cudaHostAlloc(void**, size_t, unsigned) { return cudaErrorMemoryAllocation; }
 cudaError_t cudaFuncGetAttributes(struct cudaFuncAttributes* a, const void*) { memset(a, 0, sizeof(*a)); a->numRegs = 255; return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute, int v) {
+  if (g_fail) { --g_fail; g_last = cudaErrorMemoryAllocation; return cudaErrorMemoryAllocation; }
   g_opt_in[{g_dev, f}] = (size_t)v;
   return cudaSuccess;
 }
@@ -139,17 +141,26 @@ static const Call kCalls[] = {
     {"grouped gemm wgrad", [] { return grouped(1); }},
 };
 
-int main() {
+int main(int argc, char** argv) {
+  const std::string what = argv[1];
   int wrong = 0;
   for (const Call& c : kCalls) {
     int before = 0, bad = 0;
-    for (g_dev = 0; g_dev < 3 && !bad; ++g_dev) {
-      before = g_launched;
+    if (what == "retry") {
+      g_fail = 1;
+      if (c.go() == 0) { printf("%s: the failing set-up was not seen\n", c.name); return 2; }
+      g_fail = 0;
       bad = c.go();
-      if (bad) printf("%s: %d on device %d\n", c.name, bad, g_dev);
-      if (g_launched == before) { printf("%s: no launch\n", c.name); return 2; }
+      if (bad) printf("%s: %d at the second try\n", c.name, bad);
+    } else {
+      for (g_dev = 0; g_dev < 3 && !bad; ++g_dev) {
+        before = g_launched;
+        bad = c.go();
+        if (bad) printf("%s: %d on device %d\n", c.name, bad, g_dev);
+        if (g_launched == before) { printf("%s: no launch\n", c.name); return 2; }
+      }
+      g_dev = 0;
     }
-    g_dev = 0;
     wrong += bad != 0;
   }
   return wrong;
@@ -176,5 +187,11 @@ def driver(tmp_path_factory):
 
 def test_second_device(driver):
     """A kernel that ran on one device of the process runs on the others."""
-    r = subprocess.run([str(driver)], capture_output=True, text=True, timeout=120)
+    r = subprocess.run([str(driver), "devices"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_failed_setup_is_tried_again(driver):
+    """A set-up that fails once (no memory for a moment, say) fails that call and not those after it."""
+    r = subprocess.run([str(driver), "retry"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr

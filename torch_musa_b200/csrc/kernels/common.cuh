@@ -105,19 +105,21 @@ __device__ __forceinline__ float block_max(float v, float* sh) {
 }
 
 // Set-up of a kernel that is made once: the opt-in to more than 48 KB of dynamic shared memory, and the checks beside it.  A
-// function's attributes belong to one device's copy of it, so the result is remembered per device.
+// function's attributes belong to one device's copy of it, so success is remembered per device; after a failure the next call
+// tries again.
 struct OncePerDevice {
   static constexpr int kDevices = 64;
-  std::atomic<int> result[kDevices];      // 0: not yet; otherwise the error code + 1
+  std::atomic<uint64_t> done;             // one bit per device
   template <typename F>
   int operator()(F setup) {
     int dev = 0;
     const cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    if (dev >= kDevices) return setup();
-    if (int r = result[dev].load(std::memory_order_acquire)) return r - 1;
+    const uint64_t bit = dev < kDevices ? 1ull << dev : 0;
+    if (done.load(std::memory_order_acquire) & bit) return 0;
     const int r = setup();
-    result[dev].store(r + 1, std::memory_order_release);
+    if (r == 0) done.fetch_or(bit, std::memory_order_release);
+    else (void)cudaGetLastError();        // the caller has the code: the next launch must not be blamed for it
     return r;
   }
 };
