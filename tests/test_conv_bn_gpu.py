@@ -257,3 +257,32 @@ def test_deterministic_mode(bw, dev):
         assert any("index_put" in k for k in bw.fallback_counts())
     finally:
         torch.use_deterministic_algorithms(False)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_weight_gradient_into_any_float_pointer(bw, dev, offset):
+    """The C entry takes a float pointer of any alignment (the four-wide reductions need 16 bytes)."""
+    import ctypes
+    import os
+
+    class Desc(ctypes.Structure):
+        _fields_ = [(n, ctypes.c_int64) for n in ("N", "H", "W", "C", "K", "Ho", "Wo")] + \
+                   [(n, ctypes.c_int) for n in ("R", "S", "sh", "sw", "ph", "pw", "dtype")]
+
+    lib = ctypes.CDLL(os.path.join(os.path.dirname(bw.__file__), "libb200_kernels.so"))
+    n, h, c, k = 2, 9, 24, 40
+    torch.manual_seed(offset)
+    x, dy = torch.randn(n, h, h, c).bfloat16(), torch.randn(n, h, h, k).bfloat16()
+    xd, gd = x.to(dev), dy.to(dev)
+    buf = torch.zeros(k * 9 * c + 8, device=dev)
+    d = Desc(n, h, h, c, k, h, h, 3, 3, 1, 1, 1, 1, 1)     # 3 x 3, stride 1, padding 1, bf16
+    out = buf[offset:offset + k * 9 * c]
+    rc = lib.b200_conv_wgrad(ctypes.byref(d), ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(gd.data_ptr()), ctypes.c_void_p(xd.data_ptr()),
+                             ctypes.c_void_p(bw.current_stream().cuda_stream))
+    assert rc == 0
+    bw.synchronize()
+    ref = torch.nn.grad.conv2d_weight(x.permute(0, 3, 1, 2).double(), (k, c, 3, 3), dy.permute(0, 3, 1, 2).double(), padding=1)
+    got = out.cpu().double().view(k, 3, 3, c).permute(0, 3, 1, 2)
+    # products of bf16 values are exact in fp32; sums of 162 of them
+    assert torch.allclose(got, ref, rtol=1e-4, atol=1e-4)
+    assert float(buf[:offset].abs().sum()) == 0 and float(buf[offset + k * 9 * c:].abs().sum()) == 0

@@ -352,6 +352,7 @@ conv_wgrad_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Wgr
     int acc = 0;
     uint32_t acc_phase = 0;
     const int row = q * 32 + lane;
+    const bool vec4 = (reinterpret_cast<uintptr_t>(dw) & 15) == 0;   // the rows are multiples of 32 bytes; dw is the caller's
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
       int mt, tap_i, nc, s0, s1;
       decode(tile, mt, tap_i, nc, s0, s1);
@@ -371,10 +372,16 @@ conv_wgrad_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Wgr
           const int nvalid = min(32, p.c_in - col0);   // a multiple of 8
 #pragma unroll
           for (int e = 0; e < 32; e += 4)
-            if (e < nvalid)
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(drow + c * 32 + e), "f"(__uint_as_float(raw[e])),
-                           "f"(__uint_as_float(raw[e + 1])), "f"(__uint_as_float(raw[e + 2])), "f"(__uint_as_float(raw[e + 3]))
-                           : "memory");
+            if (e < nvalid) {
+              float* o = drow + c * 32 + e;
+              if (vec4)
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o), "f"(__uint_as_float(raw[e])),
+                             "f"(__uint_as_float(raw[e + 1])), "f"(__uint_as_float(raw[e + 2])), "f"(__uint_as_float(raw[e + 3]))
+                             : "memory");
+              else
+#pragma unroll
+                for (int i = 0; i < 4; ++i) atomicAdd(o + i, __uint_as_float(raw[e + i]));
+            }
         }
       }
       tc_fence_before();
