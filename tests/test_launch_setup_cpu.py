@@ -68,7 +68,7 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char* s, void** p, unsigned, 
 static void* const A = (void*)0x10000, * const B = (void*)0x20000, * const C = (void*)0x30000, * const D = (void*)0x40000;
 
 static int rms(int dtype, int cols) {
-  return b200_rmsnorm_bwd(dtype, A, (float*)B, nullptr, C, D, A, (float*)B, C, 8, cols, nullptr);
+  return b200_rmsnorm_residual_bwd(dtype, A, (float*)B, nullptr, C, D, A, (float*)B, C, 8, cols, nullptr);
 }
 static int gemm(int m, int n, int k, int out_dtype, int in_dtype) {
   b200_gemm_desc_t g;
@@ -195,3 +195,17 @@ def test_failed_setup_is_tried_again(driver):
     """A set-up that fails once (no memory for a moment, say) fails that call and not those after it."""
     r = subprocess.run([str(driver), "retry"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_rmsnorm_bwd_keeps_its_signature(tmp_path):
+    """The kernel library is called from C and ctypes: an entry keeps its arguments, one that needs more gets a name."""
+    src = tmp_path / "sig.cpp"
+    src.write_text("""
+#include "b200_kernels.h"
+#include <type_traits>
+static_assert(std::is_same<decltype(&b200_rmsnorm_bwd), int (*)(int, void*, float*, int*, const void*, const void*, const void*, const float*,
+                                                                int64_t, int64_t, cudaStream_t)>::value, "b200_rmsnorm_bwd");
+""")
+    cxx = os.environ.get("B200_CXX", shutil.which("g++"))
+    r = subprocess.run([cxx, "-std=c++17", "-fsyntax-only", "-I", KERNELS, "-I", os.path.join(CUDA, "include"), str(src)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr

@@ -247,9 +247,9 @@ std::tuple<at::Tensor, at::Tensor> rms_norm_residual_backward(const at::Tensor& 
     at::Tensor partial = at::empty({nb, cols}, x.options().dtype(at::kFloat));
     DeviceSwitch sw(x.device().index());
     cudaStream_t s = current_raw_stream(x);
-    const int err = b200_rmsnorm_bwd(kdtype(x.scalar_type()), dx.mutable_data_ptr(), partial.data_ptr<float>(), nullptr,
-                                     g.const_data_ptr(), x.const_data_ptr(), w.const_data_ptr(), rs.data_ptr<float>(),
-                                     has_dres ? r.const_data_ptr() : nullptr, rows, cols, s);
+    const int err = b200_rmsnorm_residual_bwd(kdtype(x.scalar_type()), dx.mutable_data_ptr(), partial.data_ptr<float>(), nullptr,
+                                              g.const_data_ptr(), x.const_data_ptr(), w.const_data_ptr(), rs.data_ptr<float>(),
+                                              has_dres ? r.const_data_ptr() : nullptr, rows, cols, s);
     if (err == 0) {
       B200_KERNEL_CALL(b200_reduce_cols_sum(B200_F32, dw.mutable_data_ptr(), kdtype(dw.scalar_type()), partial.const_data_ptr(),
                                             nb, cols, s));

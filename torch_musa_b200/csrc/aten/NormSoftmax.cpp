@@ -75,7 +75,7 @@ std::tuple<at::Tensor, at::Tensor> fused_rms_norm_backward(const at::Tensor& gra
     int err = b200_rmsnorm_bwd(kdtype(x.scalar_type()), dx.mutable_data_ptr(),
                                need_dw ? partial.data_ptr<float>() : nullptr, nullptr, dy.const_data_ptr(),
                                x.const_data_ptr(), has_w ? weight->const_data_ptr() : nullptr, rs.data_ptr<float>(),
-                               nullptr, rows, cols, s);
+                               rows, cols, s);
     if (err == 0) {
       at::Tensor dw;
       if (need_dw) {

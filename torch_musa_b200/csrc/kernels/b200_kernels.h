@@ -205,8 +205,12 @@ B200_API int b200_rmsnorm_fwd(int dtype, void* y, float* rstd, const void* x, co
                               void* res_out, int64_t rows, int64_t cols, float eps, cudaStream_t stream);
 /* dx (and optionally dw partial sums in dw_partial[nblocks, cols] fp32; pass NULL to skip) */
 B200_API int b200_rmsnorm_bwd(int dtype, void* dx, float* dw_partial, int* nblocks_out_host, const void* dy,
-                              const void* x, const void* w, const float* rstd, const void* dres /* added to dx, may be
-                              NULL */, int64_t rows, int64_t cols, cudaStream_t stream);
+                              const void* x, const void* w, const float* rstd, int64_t rows, int64_t cols,
+                              cudaStream_t stream);
+/* the same with dres (may be NULL), the gradient that reaches the normalised row past the norm, added to dx */
+B200_API int b200_rmsnorm_residual_bwd(int dtype, void* dx, float* dw_partial, int* nblocks_out_host, const void* dy,
+                                       const void* x, const void* w, const float* rstd, const void* dres, int64_t rows,
+                                       int64_t cols, cudaStream_t stream);
 B200_API int b200_rmsnorm_bwd_partial_rows(int64_t rows, int64_t cols);
 B200_API int b200_layernorm_fwd(int dtype, void* y, float* mean, float* rstd, const void* x, const void* w,
                                 const void* b, int64_t rows, int64_t cols, float eps, cudaStream_t stream);

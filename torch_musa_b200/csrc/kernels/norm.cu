@@ -406,7 +406,13 @@ int b200_rmsnorm_fwd(int dtype, void* y, float* rstd, const void* x, const void*
 }
 
 int b200_rmsnorm_bwd(int dtype, void* dx, float* dw_partial, int* nblocks_out_host, const void* dy, const void* x,
-                     const void* w, const float* rstd, const void* dres, int64_t rows, int64_t cols, cudaStream_t stream) {
+                     const void* w, const float* rstd, int64_t rows, int64_t cols, cudaStream_t stream) {
+  return b200_rmsnorm_residual_bwd(dtype, dx, dw_partial, nblocks_out_host, dy, x, w, rstd, nullptr, rows, cols, stream);
+}
+
+int b200_rmsnorm_residual_bwd(int dtype, void* dx, float* dw_partial, int* nblocks_out_host, const void* dy, const void* x,
+                              const void* w, const float* rstd, const void* dres, int64_t rows, int64_t cols,
+                              cudaStream_t stream) {
   if (rows == 0) return 0;
   int nb = b200_rmsnorm_bwd_partial_rows(rows, cols);
   int rpc = (int)cdiv(rows, nb);
