@@ -225,6 +225,58 @@ def test_custom_op_sharding_rules_are_registered():
         assert getattr(torch.ops.blackwell, name).default in table, name
 
 
+def _sharded_loss_body(rank, world):
+    """The fused loss of row-sharded logits: each rank adds up its own rows, nothing is gathered."""
+    from torch.distributed.device_mesh import init_device_mesh
+    from torch.distributed.tensor import DTensor, Shard
+    from torch.distributed.tensor.debug import CommDebugMode
+    from torch_musa_b200.distributed import tensor_ops
+    from torch_musa_b200.ops.functional import _FusedCE
+
+    tensor_ops.register()
+    lib = torch.library.Library("blackwell", "IMPL", "CPU")     # plain stand-ins for the kernels
+
+    def fwd(logits, target, ignore_index=-100, label_smoothing=0.0):
+        lse = torch.logsumexp(logits, -1)
+        nll = lse - logits.gather(1, target.clamp_min(0)[:, None])[:, 0]
+        return torch.where(target == ignore_index, 0.0, nll), lse
+
+    def mean(loss_rows, target, ignore_index=-100):
+        n = (target != ignore_index).sum().clamp_min(1).float()
+        return loss_rows.sum() / n, n
+
+    def bwd(logits, lse, target, grad_loss, scale, ignore_index, label_smoothing):
+        g = torch.exp(logits - lse[:, None])
+        g[torch.arange(len(target)), target.clamp_min(0)] -= 1
+        return g * (target != ignore_index)[:, None] * grad_loss * scale
+
+    lib.impl("cross_entropy_fwd", fwd)
+    lib.impl("cross_entropy_mean", mean)
+    lib.impl("cross_entropy_bwd", bwd)
+    mesh = init_device_mesh("cpu", (world,))
+    torch.manual_seed(0)
+    logits, target = torch.randn(6 * world, 11), torch.randint(0, 11, (6 * world,))
+    target[1:4] = -100                                     # the ranks count different numbers of rows
+    rows = slice(6 * rank, 6 * rank + 6)
+    x = DTensor.from_local(logits[rows].clone().requires_grad_(), mesh, [Shard(0)])
+    x.retain_grad()
+    t = DTensor.from_local(target[rows].clone(), mesh, [Shard(0)])
+    with CommDebugMode() as comm:
+        loss = _FusedCE.apply(x, t, -100, 0.0, "mean", False)
+    gathers = [n for op, n in comm.get_comm_counts().items() if "gather" in str(op)]
+    assert not sum(gathers), comm.get_comm_counts()
+    ref_x = logits.clone().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(ref_x, target)
+    ref.backward()
+    loss.backward()
+    assert torch.allclose(loss.full_tensor(), ref.detach(), rtol=1e-6)
+    assert torch.allclose(x.grad.full_tensor(), ref_x.grad, rtol=1e-5, atol=1e-7)
+
+
+def test_fused_loss_of_sharded_rows_gathers_nothing():
+    run_ranks(_sharded_loss_body, 2, "gloo")
+
+
 def _tp_decode_body(rank, world):
     import copy
     from torch_musa_b200.models import Llama, llama_tiny_config

@@ -7,6 +7,11 @@ from typing import List, Optional, Tuple
 import torch
 import torch.nn.functional as F
 
+try:
+    from torch.distributed.tensor import DTensor
+except Exception:  # pragma: no cover  (torch built without distributed)
+    DTensor = None
+
 
 def _on_device(t: torch.Tensor) -> bool:
     return t.device.type == "blackwell"
@@ -275,13 +280,22 @@ def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 
 # ------------------------------------------------------------------------- cross entropy
+def _mean_of_counted(loss_rows, target, ignore_index):
+    """(mean over the rows that count, their number), in one launch.  Row shards are added up where they are instead: the
+    one-launch operation would have to gather losses and targets first."""
+    if DTensor is not None and isinstance(loss_rows, DTensor):
+        n = (target != ignore_index).sum().clamp_min(1).to(torch.float32)
+        return loss_rows.sum() / n, n
+    return torch.ops.blackwell.cross_entropy_mean(loss_rows, target, ignore_index)
+
+
 class _FusedCE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, target, ignore_index, label_smoothing, reduction, inplace_backward):
         loss_rows, lse = torch.ops.blackwell.cross_entropy_fwd(logits, target, ignore_index, label_smoothing)
         n_valid = None
         if reduction == "mean":
-            out, n_valid = torch.ops.blackwell.cross_entropy_mean(loss_rows, target, ignore_index)
+            out, n_valid = _mean_of_counted(loss_rows, target, ignore_index)
         elif reduction == "sum":
             out = loss_rows.sum()
         else:
