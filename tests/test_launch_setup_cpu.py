@@ -1,6 +1,7 @@
 """Set-up of the kernels that take more than 48 KB of shared memory, against a fake CUDA runtime (no GPU): the opt-in belongs
 to one device's copy of a function, so every device needs its own."""
 import os
+import re
 import shutil
 import subprocess
 
@@ -209,3 +210,17 @@ static_assert(std::is_same<decltype(&b200_rmsnorm_bwd), int (*)(int, void*, floa
     cxx = os.environ.get("B200_CXX", shutil.which("g++"))
     r = subprocess.run([cxx, "-std=c++17", "-fsyntax-only", "-I", KERNELS, "-I", os.path.join(CUDA, "include"), str(src)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+def test_blocks_that_gave_up_wait_for_their_copies():
+    """Every kernel with tensor memory ends in settle_abort, after its last barrier: a block that gave up on a wait must not
+    release shared memory that its copies in flight still write."""
+    seen = 0
+    for name in sorted(os.listdir(KERNELS)):
+        if name.endswith(".cu"):
+            text = open(os.path.join(KERNELS, name)).read()
+            ends = re.findall(r"__syncthreads\(\);(?:(?!__syncthreads).)*?settle_abort\(", text, re.S)
+            calls = re.findall(r"^ +tmem_dealloc(?:_pair)?\(", text, re.M)
+            assert len(ends) == len(calls), name
+            seen += len(calls)
+    assert seen >= 8

@@ -464,16 +464,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
   }
 
-  // a CTA that gave up on a wait may still have tile loads in flight towards its shared memory: give them a bounded moment
-  if (*abort_flag && threadIdx.x == 0)
-    for (int i = 0; i < 200; ++i) __nanosleep(1000);
   tc_fence_before();
   __syncthreads();
   if (warp == 13) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kBwdTmemCols);
   }
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
+  settle_abort(abort_flag, p.status);
 }
 
 bool make_dq_map(CUtensorMap* out, float* ptr, int64_t rows) {

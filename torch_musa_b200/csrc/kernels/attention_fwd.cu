@@ -370,7 +370,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     tc_fence_after();
     tmem_dealloc(tmem_base, kAttnTmemCols);
   }
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
+  settle_abort(abort_flag, p.status);
 }
 
 template <typename K>

@@ -118,7 +118,7 @@ __device__ __forceinline__ void teardown(const Smem& s, uint32_t tmem_base, int 
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
-  if (threadIdx.x == 0 && *s.abort_flag && status) atomicExch(status, 1);
+  settle_abort(s.abort_flag, status);
 }
 
 // MMA issue for one pipeline stage: four K=16 steps.

@@ -56,6 +56,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
+// Called by every thread after the block's last barrier.  A block that gave up on a wait may still have copies in flight
+// towards its shared memory: thread 0 keeps that memory for a bounded moment, in which they land, and sets the status word.
+// (After the barrier, because before it another warp's wait may not have run out yet.)
+__device__ __forceinline__ void settle_abort(volatile int* abort_flag, int* status) {
+  if (threadIdx.x == 0 && *abort_flag) {
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    if (status) atomicExch(status, 1);
+  }
+  __syncwarp();
+}
+
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1,
                                             int c2) {
   asm volatile(

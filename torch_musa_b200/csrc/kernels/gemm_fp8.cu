@@ -247,16 +247,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
   }
 
-  // a CTA that gave up on a wait may still have tile loads in flight towards its shared memory
-  if (*abort_flag && threadIdx.x == 0)
-    for (int i = 0; i < 200; ++i) __nanosleep(1000);
   tc_fence_before();
   __syncthreads();
   if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem_base, C::kTmemCols);
   }
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
+  settle_abort(abort_flag, p.status);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

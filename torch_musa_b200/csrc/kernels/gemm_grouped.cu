@@ -262,7 +262,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
+  settle_abort(abort_flag, p.status);
 }
 
 template <typename OutT, bool RAGGED_K, bool B_KMAJOR>

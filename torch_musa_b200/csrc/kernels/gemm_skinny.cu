@@ -202,16 +202,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // a peer may still read this CTA's sums
   }
 
-  // a CTA that gave up on a wait may still have tile loads in flight towards its shared memory
-  if (*abort_flag && threadIdx.x == 0)
-    for (int i = 0; i < 200; ++i) __nanosleep(1000);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, C::kTmemCols);
   }
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
+  settle_abort(abort_flag, p.status);
 }
 
 template <typename OutT, int MP>

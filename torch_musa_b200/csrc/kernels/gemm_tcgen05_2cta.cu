@@ -632,19 +632,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   }
 
-  // A CTA that gave up on a wait may still have tile loads in flight towards its shared memory: give them
-  // a bounded moment to land before the memory is released.
-  if (*abort_flag && threadIdx.x == 0) {
-    for (int i = 0; i < 200; ++i) __nanosleep(1000);
-  }
   tc_fence_before();
   __syncthreads();
+  settle_abort(abort_flag, p.status);
   cluster_sync_all();  // no CTA of the pair leaves while the other may still signal it
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kTmemCols);
   }
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
 }
 
 // ------------------------------------------------------------------ host side
