@@ -435,8 +435,9 @@ def test_fused_cross_entropy_row_widths(bw, dev, rows, cols, dt):
     assert float(none) == 0.0
 
 
-# One aligned 16-byte group, a whole half, and all of the row at a finite mask value; logits far from zero.
-@pytest.mark.parametrize("rows,cols", [(6, 1024), (6, 4096), (6, 32000), (1300, 1024), (700, 4104)])
+# One aligned 16-byte group, a whole half, and all of the row at a finite mask value; logits far from zero; each number of threads
+# per row, with and without vector loads.
+@pytest.mark.parametrize("rows,cols", [(6, 1024), (6, 4096), (6, 32000), (1300, 1024), (700, 4104), (320, 2056), (2500, 1032), (2500, 1001), (1200, 901)])
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_row_statistics_masked_and_offset(bw, dev, dt, rows, cols):
     from torch_musa_b200.ops import fused_cross_entropy

@@ -9,6 +9,8 @@
 // csrc/extension/FusedCrossEntropyLoss.mu:55,160,293 (vocab-parallel pieces).
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace b200k {
 namespace {
 
@@ -54,14 +56,21 @@ __device__ __forceinline__ float exp2f_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// ((x0, x1) - m) * log2(e), two fp32 operations per instruction
+__device__ __forceinline__ void log2_ratio(float& d0, float& d1, float x0, float x1, float m) {
+  asm("{\n\t.reg .b64 rx, rm, rs, rd;\n\t"
+      "mov.b64 rx, {%2, %3};\n\tmov.b64 rm, {%4, %4};\n\tmov.b64 rs, {%5, %5};\n\t"
+      "add.rn.f32x2 rd, rx, rm;\n\tmul.rn.f32x2 rd, rd, rs;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d0), "=f"(d1)
+      : "f"(x0), "f"(x1), "f"(-m), "f"(1.4426950408889634f));
+}
 
 // N vectors of a row into the running (maximum, sum): the maximum in four chains, one correction of the sum, then the
 // exponentials in four chains of additions.  The maximum is subtracted before the scaling by log2(e): rounded on its own,
 // the product m * log2(e) would put its error, or for masks near the type's lowest value its overflow, into every term.
 template <int N, typename T>
-__device__ __forceinline__ void ms_push_vecs(MaxSum& acc, const Vec16<T> (&v)[N]) {
+__device__ __forceinline__ void ms_push_vecs(MaxSum& acc, const Vec16<T>* v) {
   constexpr int V = Vec16<T>::N;
-  constexpr float kLog2e = 1.4426950408889634f;
   float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
   for (int u = 0; u < N; ++u)
@@ -74,7 +83,12 @@ __device__ __forceinline__ void ms_push_vecs(MaxSum& acc, const Vec16<T> (&v)[N]
 #pragma unroll
   for (int u = 0; u < N; ++u)
 #pragma unroll
-    for (int k = 0; k < V; ++k) sm[k & 3] += exp2f_approx((ToF<T>::to(v[u].v[k]) - acc.m) * kLog2e);
+    for (int k = 0; k < V; k += 2) {
+      float d0, d1;
+      log2_ratio(d0, d1, ToF<T>::to(v[u].v[k]), ToF<T>::to(v[u].v[k + 1]), acc.m);
+      sm[k & 3] += exp2f_approx(d0);
+      sm[(k & 3) + 1] += exp2f_approx(d1);
+    }
   acc.s += (sm[0] + sm[1]) + (sm[2] + sm[3]);
 }
 
@@ -84,27 +98,29 @@ __device__ __forceinline__ MaxSum row_stats(const T* __restrict__ xr, int64_t co
   constexpr int V = Vec16<T>::N;
   MaxSum acc{-INFINITY, 0.f};
   if constexpr (VEC) {
-    // Four 16-byte loads per thread are in flight while the four before them are worked on.
-    const int nvec = (int)(cols / V), step = blockDim.x * 4;
-    Vec16<T> cur[4], nxt[4];
-    auto load = [&](Vec16<T>(&v)[4], int i0) {
+    // A group of 16 elements per thread is on its way while the one before it is worked on.  (Groups of 32 16-bit elements took
+    // 96 registers, which leaves room for 640 threads on an SM.)
+    constexpr int U = 16 / V;
+    const int nvec = (int)(cols / V), step = blockDim.x * U;
+    Vec16<T> cur[U], nxt[U];
+    auto load = [&](Vec16<T>(&v)[U], int i0) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * blockDim.x;
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * (int)blockDim.x;
         if (i < nvec) v[u] = ld16(xr + (int64_t)i * V);
       }
     };
-    load(cur, threadIdx.x);
     int i0 = threadIdx.x;
-    for (; i0 - (int)threadIdx.x + step <= nvec; i0 += step) {     // whole groups: every thread has four vectors
+    load(cur, i0);
+    for (; i0 - (int)threadIdx.x + step <= nvec; i0 += step) {     // whole groups: every thread has U vectors
       load(nxt, i0 + step);
-      ms_push_vecs<4>(acc, cur);
+      ms_push_vecs<U>(acc, cur);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) cur[u] = nxt[u];
+      for (int u = 0; u < U; ++u) cur[u] = nxt[u];
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (i0 + u * (int)blockDim.x < nvec) ms_push_vecs<1>(acc, reinterpret_cast<const Vec16<T>(&)[1]>(cur[u]));
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * (int)blockDim.x < nvec) ms_push_vecs<1>(acc, cur + u);
   } else {
     for (int64_t i = threadIdx.x; i < cols; i += blockDim.x) ms_push(acc, ToF<T>::to(xr[i]));
   }
@@ -112,7 +128,7 @@ __device__ __forceinline__ MaxSum row_stats(const T* __restrict__ xr, int64_t co
 }
 
 template <typename T, bool VEC, bool LOG>
-__global__ void __launch_bounds__(kThreads) softmax_fwd_kernel(T* __restrict__ y, const T* __restrict__ x, int64_t cols) {
+__global__ void __launch_bounds__(kThreads, 2) softmax_fwd_kernel(T* __restrict__ y, const T* __restrict__ x, int64_t cols) {
   constexpr int V = Vec16<T>::N;
   __shared__ float shm[32], shs[32];
   const int64_t row = blockIdx.x;
@@ -161,7 +177,7 @@ __global__ void __launch_bounds__(kThreads) softmax_bwd_kernel(T* __restrict__ d
 }
 
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(kThreads) ce_fwd_kernel(float* __restrict__ loss, float* __restrict__ lse_out,
+__global__ void __launch_bounds__(kThreads, 2) ce_fwd_kernel(float* __restrict__ loss, float* __restrict__ lse_out,
                                                           const T* __restrict__ logits,
                                                           const int64_t* __restrict__ target, int64_t cols,
                                                           int64_t ignore_index, float smoothing) {
@@ -268,7 +284,7 @@ __global__ void __launch_bounds__(1024) ce_mean_kernel(float* __restrict__ mean,
 }
 
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(kThreads) online_stats_kernel(float* __restrict__ stats3,
+__global__ void __launch_bounds__(kThreads, 2) online_stats_kernel(float* __restrict__ stats3,
                                                                 const T* __restrict__ logits,
                                                                 const int64_t* __restrict__ target, int64_t cols,
                                                                 int64_t vocab_start) {
@@ -311,11 +327,49 @@ __global__ void __launch_bounds__(kThreads) vp_ce_finish_kernel(float* __restric
   }
 }
 
-// Threads per row.  A row's blocks end in a reduction and a few dependent scalar operations during which the block loads
-// nothing; many small blocks per SM at different points of their rows keep memory busy.  With few rows the row has to be
-// spread over more threads instead.  4096 x 32000 bf16 at 128 / 256 / 512 threads: forward 70 / 79 / 131 us (92 before, with
-// 512 threads and one chain of maxima and sums), backward 88 / 92 / 102 us.
-inline int row_threads(int64_t rows) { return rows >= kSMs * 8 ? 128 : (rows >= kSMs * 4 ? 256 : kThreads); }
+// ---- threads per row
+// Vector loads.  A row's block ends in a reduction and a few dependent scalar operations during which it loads nothing, so many
+// small blocks per SM at different points of their rows keep memory busy; with few rows a row has to be spread over more threads
+// instead.  From 16 rows per SM on 64 threads are enough for short rows, and for fp32, where a thread's group is twice the bytes.
+// Row statistics, 64 / 128 / 256 / 512 threads: 4096 x 32000 bf16 58 / 55 / 62 / 75 us, fp32 85 / 86 / 84 / 94, x 50304 fp32 124 /
+// 129 / 125 / 134, x 8192 bf16 18 / 20 / 27 / 42; 1184 x 32000 bf16 24 / 19 / 21 / 24; 600 x 32000 22 / 14.3 / 15.4 / 15.5; 32 x
+// 32000 12 / 7.4 / 5.2 / 4.6.  (4096 x 32000 bf16 took 89 us with 512 threads and one chain of maxima and sums.)
+inline int vec_threads(int64_t rows, int64_t cols, int elem) {
+  const bool small = elem == 4 || cols * elem < 24 * 1024;
+  int t = rows >= kSMs * 16 && small ? 64 : rows >= kSMs * 4 ? 128 : rows >= kSMs * 2 ? 256 : kThreads;
+  while (t > 32 && (int64_t)t * 4 >= cols) t /= 2;
+  return t;
+}
+// Element by element (ragged or misaligned rows) a thread is a chain of dependent exponentials: the time is the number of waves
+// of blocks times what one block takes, a fixed part worth about six elements and its share of the row.  1184 x 50257 at 128 /
+// 256 / 512 threads: 209 / 110 / 115 us; 4096 x 50257: 413 / 417 / 388; 4096 x 4001: 43 / 46 / 52.
+inline int scalar_threads(int64_t rows, int64_t cols) {
+  int best = kThreads;
+  double best_cost = 1e300;
+  for (int t = kThreads; t >= 64; t /= 2) {
+    const double cost = (double)cdiv(rows * t, (int64_t)kSMs * 2048) * (6.0 + (double)cols / t);
+    if (cost <= best_cost) { best = t; best_cost = cost; }
+  }
+  return best;
+}
+inline int stats_threads(bool vec, int64_t rows, int64_t cols, int elem) {
+  return vec ? vec_threads(rows, cols, elem) : scalar_threads(rows, cols);
+}
+// The second pass of a softmax reads its row again: with a thread per 256 bytes the rows in flight (1024 threads per SM) are 38 MB
+// and come from L2.  4096 x 32000 at 128 / 256 / 512 threads: bf16 135 / 115 / 131 us, fp32 248 / 220 / 178.
+inline int softmax_threads(bool vec, int64_t rows, int64_t cols, int elem) {
+  int t = stats_threads(vec, rows, cols, elem);
+  if (!vec || rows >= kSMs * 4)
+    while (t < kThreads && (int64_t)t * 256 < cols * elem) t *= 2;
+  return t;
+}
+// The loss's gradient streams in and out; rows of 112 KB and more keep whole blocks.  4096 x 32000 at 128 / 256 / 512 threads:
+// bf16 91 / 93 / 104 us, fp32 172 / 164 / 162; 1184 x 50257 fp32 110 / 97 / 94.
+inline int ce_bwd_threads(bool vec, int64_t rows, int64_t cols, int elem) {
+  if (cols * elem >= 112 * 1024) return kThreads;
+  if (!vec) return std::max(128, scalar_threads(rows, cols));
+  return rows >= kSMs * 8 ? 128 : rows >= kSMs * 4 ? 256 : kThreads;
+}
 
 }  // namespace
 }  // namespace b200k
@@ -330,12 +384,13 @@ int b200_softmax_fwd(int dtype, void* y, const void* x, int64_t rows, int64_t co
   B200K_DISPATCH_FLOAT(dtype, T, {
     bool vec = cols % Vec16<T>::N == 0 && aligned16((const T*)x) && aligned16((T*)y);
     dim3 grid((unsigned)rows);
+    const int threads = softmax_threads(vec, rows, cols, (int)sizeof(T));
     if (vec) {
-      if (log_softmax) softmax_fwd_kernel<T, true, true><<<grid, kThreads, 0, stream>>>((T*)y, (const T*)x, cols);
-      else softmax_fwd_kernel<T, true, false><<<grid, kThreads, 0, stream>>>((T*)y, (const T*)x, cols);
+      if (log_softmax) softmax_fwd_kernel<T, true, true><<<grid, threads, 0, stream>>>((T*)y, (const T*)x, cols);
+      else softmax_fwd_kernel<T, true, false><<<grid, threads, 0, stream>>>((T*)y, (const T*)x, cols);
     } else {
-      if (log_softmax) softmax_fwd_kernel<T, false, true><<<grid, kThreads, 0, stream>>>((T*)y, (const T*)x, cols);
-      else softmax_fwd_kernel<T, false, false><<<grid, kThreads, 0, stream>>>((T*)y, (const T*)x, cols);
+      if (log_softmax) softmax_fwd_kernel<T, false, true><<<grid, threads, 0, stream>>>((T*)y, (const T*)x, cols);
+      else softmax_fwd_kernel<T, false, false><<<grid, threads, 0, stream>>>((T*)y, (const T*)x, cols);
     }
     B200K_LAUNCH_RET();
   })
@@ -360,7 +415,7 @@ int b200_cross_entropy_fwd(int dtype, float* loss, float* lse, const void* logit
   B200K_DISPATCH_FLOAT(dtype, T, {
     bool vec = cols % Vec16<T>::N == 0 && aligned16((const T*)logits);
     dim3 grid((unsigned)rows);
-    const int threads = row_threads(rows);
+    const int threads = stats_threads(vec, rows, cols, (int)sizeof(T));
     if (vec) ce_fwd_kernel<T, true><<<grid, threads, 0, stream>>>(loss, lse, (const T*)logits, target, cols, ignore_index, label_smoothing);
     else ce_fwd_kernel<T, false><<<grid, threads, 0, stream>>>(loss, lse, (const T*)logits, target, cols, ignore_index, label_smoothing);
     B200K_LAUNCH_RET();
@@ -382,8 +437,9 @@ int b200_cross_entropy_bwd(int dtype, void* dlogits, const void* logits, const f
   B200K_DISPATCH_FLOAT(dtype, T, {
     bool vec = cols % Vec16<T>::N == 0 && aligned16((const T*)logits) && aligned16((T*)dlogits);
     dim3 grid((unsigned)rows);
-    if (vec) ce_bwd_kernel<T, true><<<grid, row_threads(rows), 0, stream>>>((T*)dlogits, (const T*)logits, lse, target, grad_loss, grad_is_scalar, scale, cols, ignore_index, label_smoothing);
-    else ce_bwd_kernel<T, false><<<grid, row_threads(rows), 0, stream>>>((T*)dlogits, (const T*)logits, lse, target, grad_loss, grad_is_scalar, scale, cols, ignore_index, label_smoothing);
+    const int threads = ce_bwd_threads(vec, rows, cols, (int)sizeof(T));
+    if (vec) ce_bwd_kernel<T, true><<<grid, threads, 0, stream>>>((T*)dlogits, (const T*)logits, lse, target, grad_loss, grad_is_scalar, scale, cols, ignore_index, label_smoothing);
+    else ce_bwd_kernel<T, false><<<grid, threads, 0, stream>>>((T*)dlogits, (const T*)logits, lse, target, grad_loss, grad_is_scalar, scale, cols, ignore_index, label_smoothing);
     B200K_LAUNCH_RET();
   })
   return (int)cudaErrorNotSupported;
@@ -395,8 +451,9 @@ int b200_online_softmax_stats(int dtype, float* stats3, const void* logits, cons
   B200K_DISPATCH_FLOAT(dtype, T, {
     bool vec = cols % Vec16<T>::N == 0 && aligned16((const T*)logits);
     dim3 grid((unsigned)rows);
-    if (vec) online_stats_kernel<T, true><<<grid, kThreads, 0, stream>>>(stats3, (const T*)logits, target, cols, vocab_start);
-    else online_stats_kernel<T, false><<<grid, kThreads, 0, stream>>>(stats3, (const T*)logits, target, cols, vocab_start);
+    const int threads = stats_threads(vec, rows, cols, (int)sizeof(T));
+    if (vec) online_stats_kernel<T, true><<<grid, threads, 0, stream>>>(stats3, (const T*)logits, target, cols, vocab_start);
+    else online_stats_kernel<T, false><<<grid, threads, 0, stream>>>(stats3, (const T*)logits, target, cols, vocab_start);
     B200K_LAUNCH_RET();
   })
   return (int)cudaErrorNotSupported;
