@@ -100,7 +100,7 @@ def test_scaled_mm_tiles(bw, dev, m, n, k, out_dtype):
 
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize("rows,k", [(1, 128), (5, 1152), (67, 4096)])
+@pytest.mark.parametrize("rows,k", [(1, 128), (5, 1152), (67, 4096), (520, 4224)])
 def test_quantize_routes_agree(bw, dev, dt, rows, k):
     """The vectorised quantiser and the one for any alignment give the same bytes and scales."""
     torch.manual_seed(rows)
