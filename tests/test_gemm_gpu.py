@@ -231,7 +231,7 @@ def test_grouped_gemm_device_side_counts(bw, dev, counts, R):
 
 
 @pytest.mark.parametrize("m", [1, 15, 17, 33, 64])
-@pytest.mark.parametrize("n,k", [(64, 256), (1000, 328), (4096, 4096), (129, 2048), (20008, 264), (24, 512)])
+@pytest.mark.parametrize("n,k", [(64, 256), (1000, 328), (1000, 648), (4096, 4096), (129, 2048), (20008, 264), (20008, 2056), (24, 512)])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 def test_few_rows(bw, dev, m, n, k, dt):
     """The few-row kernel at the edges of its row paddings, with remainders of N (also ones that rule out vector stores) and K,

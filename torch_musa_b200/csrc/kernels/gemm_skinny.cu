@@ -7,13 +7,14 @@
 // partial products through global memory and a second kernel.  Here the operands change places: 128 rows of B are the M128
 // operand and the rows of A, padded to 16 / 32 / 64, the N operand, so a stage of the ring is 16 KB of B and 2 to 8 KB of A.
 // K is cut over the CTAs of a cluster until about two CTAs per SM stream B together (each has half of an SM's shared memory
-// as its ring, 190 KB per SM in flight); they all are resident at once, share the memory's bandwidth evenly and end together,
-// so an uneven number of CTAs per SM does not matter.  The cluster adds its partial sums over distributed shared memory in
-// rank order (the result does not depend on timing), each CTA a share of the rows of A.
+// as its ring, 190 KB per SM in flight): while the CTAs are no more than two per SM they all are resident, share the memory's
+// bandwidth and end together, so an uneven number per SM does not matter.  From 130 tiles of B on K stays whole, with 130 to 148
+// tiles there is less than one CTA per SM (n = 16512 27.1 us, 16640 28.9, still ahead of the general kernel's 34), and past 296
+// tiles a second wave begins (n = 37888 53.0 us, 38016 64.0 against 74.0).  The cluster adds its partial sums over distributed
+// shared memory in rank order (the result does not depend on timing), each CTA a share of the rows of A.
 // What bounds it: memory, and for small products the launch, the ring's first fill and the epilogue (about 5 us).  Streams of
-// products with weights out of L2, M = 32, general kernel with split-K -> this one: 12288 x 4096 30.8 -> 24.4 us (4.1 TB/s),
-// 22016 x 4096 39.7 -> 36.6 (4.9), 4096 x 11008 25.0 -> 22.7, 32000 x 4096 50.1 -> 48.4 (5.4), 6144 x 4096 20.7 -> 16.4,
-// 512 x 4096 14.4 -> 8.2.
+// products with weights out of L2, K = 4096, M = 32, general kernel with split-K -> this one: n = 12288 27.8 -> 22.2 us (4.5
+// TB/s), 22016 37.7 -> 34.8 (5.2), 32000 47.7 -> 45.5 (5.8), 6144 18.5 -> 14.4, 512 9.9 -> 7.0.
 // Waits are bounded as in the dense kernel; every thread takes part in both cluster barriers whatever happened before.
 //
 // Parity: the reference sends mm/addmm to a closed vendor library (reference torch_musa/csrc/aten/ops/Matmul.cpp:293-335).
@@ -258,14 +259,22 @@ int by_rows(const b200_gemm_desc_t* g, void* d, const void* a, const void* b, in
 
 }  // namespace
 
-// The line: up to 64 rows (N operand of the instruction; at 64 rows 12288 x 4096 takes 26.9 us against 37.1, 22016 x 4096 39.1
-// against 40.4), and K long enough that the ring is more than its first fill (K = 128: 7.7 us against 6.6 at 64 rows; from 256
-// on never slower, 64 to 50257 columns).  Few columns with a very long K stay with the general kernel, whose split-K is not
-// limited to the eight CTAs of a cluster.
+// The line: up to 64 rows (N operand of the instruction) and K long enough to pay for the ring's first fill and the epilogue,
+// which grows with the rows, is not overlapped with another tile and in a second wave is paid twice.  General kernel -> this
+// one: 64 x 64 x 256 5.1 -> 6.7 us, x 768 7.5 -> 8.0; 64 x 12288 x 512 9.9 -> 10.6, x 768 11.4 -> 11.0; 64 x 28672 x 1024 15.9 ->
+// 16.3, x 3072 34.6 -> 34.4; 64 x 38016 x 2048 39.2 -> 40.1, x 3072 55.9 -> 55.3; 48 x 38016 x 1024 22.2 -> 23.3; 32 x 38016 x
+// 512 13.7 -> 15.0, x 1024 22.9 -> 22.0; up to 16 rows never slower from K = 256 on (128: 6.6 -> 7.7).  Few columns with a very
+// long K stay with the general kernel, whose split-K is not limited to the eight CTAs of a cluster.
 bool gemm_skinny_fits(const b200_gemm_desc_t* g) {
-  return g->m <= 64 && std::max(g->batch, 1) == 1 && g->a_kmajor && g->b_kmajor && g->in_dtype != B200_F32 && g->n >= 64 &&
-         g->k >= 256 &&
-         (g->n >= 2048 || g->k <= 8192);
+  if (g->m > 64 || std::max(g->batch, 1) != 1 || !g->a_kmajor || !g->b_kmajor || g->in_dtype == B200_F32 || g->n < 64) return false;
+  const int tiles = (g->n + BN - 1) / BN, sms = gemm_sm_count();
+  const bool waves = tiles > 2 * sms;
+  int k_min = 256;
+  if (tiles == 1) k_min = g->m > 48 ? 1024 : g->m > 32 ? 768 : g->m > 16 ? 512 : 256;
+  else if (g->m > 48) k_min = waves ? 3072 : tiles > sms ? 2048 : tiles > sms / 2 ? 768 : 512;
+  else if (g->m > 32) k_min = waves ? 2048 : tiles > sms / 2 ? 768 : 256;
+  else if (g->m > 16) k_min = waves ? 1024 : 256;
+  return g->k >= k_min && (g->n >= 2048 || g->k <= 8192);
 }
 
 int gemm_launch_skinny(const b200_gemm_desc_t* g, void* d, const void* a, const void* b, cudaStream_t stream) {
