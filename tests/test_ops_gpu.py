@@ -410,6 +410,22 @@ def test_rms_norm_residual_backward(bw, dev, rows, cols, dt, with_residual_grad)
     assert bw._C._gemm_status(False) == 0
 
 
+def test_rms_norm_residual_second_order_is_refused(bw, dev):
+    """create_graph gives the same first-order gradients; differentiating them again says that it is not supported."""
+    from torch_musa_b200.ops import rms_norm_residual
+
+    torch.manual_seed(0)
+    x, r, w = (torch.randn(s, device=dev, requires_grad=True) for s in ((4, 64), (4, 64), (64,)))
+    y, h = rms_norm_residual(x, r, w, 1e-5)
+    gs = [torch.randn_like(y).detach(), torch.randn_like(h).detach()]
+    first = torch.autograd.grad([y, h], [x, r, w], gs, retain_graph=True)
+    again = torch.autograd.grad([y, h], [x, r, w], gs, create_graph=True)
+    for a, b in zip(first, again):
+        assert torch.allclose(a, b, rtol=1e-5, atol=1e-6)     # fp32 sums of 64 and 4 terms in another order
+    with pytest.raises(RuntimeError, match="not implemented"):
+        torch.autograd.grad(sum(t.square().sum() for t in again), [x, r, w])
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 8), (5, 4001), (700, 520), (1300, 4104), (1200, 32000)])
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_fused_cross_entropy_row_widths(bw, dev, rows, cols, dt):

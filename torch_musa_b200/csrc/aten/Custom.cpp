@@ -262,8 +262,7 @@ std::tuple<at::Tensor, at::Tensor> rms_norm_residual_backward(const at::Tensor& 
 }
 
 // Autograd of rms_norm_residual in C++: the operation is called once per sub-layer on rows that take a few microseconds, and
-// the interpreter's part of a Python autograd function was most
-// of a call (32 x 4096 rows without gradients: 13.1 us a call
+// the interpreter's part of a Python autograd function was most of a call (32 x 4096 rows without gradients: 13.1 us a call
 // before, 8.4 now; 4096 x 4096 with both directions: 95 us against 55 us of kernels before, 87 now).
 using RmsResidualOut = std::tuple<at::Tensor, at::Tensor, at::Tensor>;
 RmsResidualOut call_rms_norm_residual(const at::Tensor& x, const at::Tensor& residual, const at::Tensor& weight, double eps) {
@@ -288,7 +287,9 @@ class RmsNormResidualFn : public torch::autograd::Function<RmsNormResidualFn> {
     const at::Tensor &res = saved[0], &weight = saved[1], &rstd = saved[2];
     const at::Tensor dy = grads[0].defined() ? grads[0] : at::zeros_like(res);
     at::Tensor dx, dw;
-    if (at::GradMode::is_enabled()) {     // gradients of the gradients: the composition that autograd can follow
+    // Second order is not supported.  With create_graph the gradients come from an operation whose node says so when it is
+    // differentiated; the one below has no autograd of its own, so its outputs would pass for constants.
+    if (at::GradMode::is_enabled()) {
       std::tie(dx, dw) = at::_fused_rms_norm_backward(dy.contiguous(), res, {res.size(-1)}, rstd, weight, {true, true});
       if (grads[1].defined()) dx = at::add(dx, grads[1]);
     } else {
