@@ -241,9 +241,17 @@ def test_backward_edges(bw, dev, native_sdp, Sq, Sk, H, Hkv, causal):
     out.backward(g.to(dev))
     assert bw._C._native_sdp_backward_calls() == before + 1
     for name, a, b in (("dq", qd.grad, qr.grad), ("dk", kd.grad, kr.grad), ("dv", vd.grad, vr.grad)):
+        a = a.float().cpu()
+        if Sq == 1 and Sk == 1 and name != "dv":     # the softmax is constant: rounding noise of the two sums that cancel
+            assert a.abs().max() < 3e-2, name
+            continue
         # P and dS are rounded to bf16 (2^-9) before they are multiplied, the result is rounded again: 3e-2 of the largest entry
-        # as above; an exact zero everywhere (one query and one key: the softmax is constant) may come out as rounding noise
-        err = (a.float().cpu() - b).abs().max()
-        assert err < 3e-2 * max(float(b.abs().max()), 1.0), (name, float(err))
+        # as above
+        err = (a - b).abs().max()
+        assert err < 3e-2 * b.abs().max(), (name, float(err))
+        # and for every block of 128 rows by itself, in the 2-norm: those two roundings, the output's in delta, and the
+        # cancellation in dP - delta come to a few times 2^-9; rows that no query sees are exact zeros
+        for i, (ab, bb) in enumerate(zip(a.split(128, 2), b.split(128, 2))):
+            assert (ab - bb).norm() <= 8 * 2.0 ** -9 * bb.norm(), (name, i, float((ab - bb).norm() / bb.norm()))
     bw.synchronize()
     assert bw._C._gemm_status(False) == 0
