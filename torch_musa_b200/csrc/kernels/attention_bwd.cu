@@ -21,10 +21,11 @@
 // next dP^T -> next dS.  P^T in TMEM instead of shared memory pays for the separate staging boxes.  Q streams through two
 // slots, dO through one (it is free after dV), lse and delta through a two-slot ring filled by a warp of its own; every wait
 // is bounded.
-// What bounds it now is shared memory: per pair the products read 288 KB, the tiles of Q and dO bring 64, dS^T 32 and the
-// staged dQ 128, which at 128 bytes per clock is 4000 clocks beside 2560 of products (4400 measured, at 32 heads x 4096 x
-// 128).  bf16, before -> after: causal 672 -> 351 us (980 TFLOP/s), full 1310 -> 640.  Registers: 96 for the warps that
-// issue keep their descriptors out of local memory, whose traffic goes through the same shared-memory path (with 56: +9 %).
+// What bounds it now is shared memory: per pair an SM spends 5060 clocks, the starts and ends of its CTAs included; the products
+// read 2300 wavefronts of 128 bytes (288 KB) and the threads' loads and stores (dS^T, the staged dQ, lse and delta) take 2840
+// more, 1290 of them without the conflicts, while the tensor core is busy for 2560 (counters at 32 heads x 4096 x 128).  bf16,
+// before -> after: causal 672 -> 351 us (980 TFLOP/s), full 1310 -> 640.  Registers: 96 for the warps that issue keep their
+// descriptors out of local memory, whose traffic goes through the same shared-memory path (with 56: +9 %).
 // Tried and not kept: starting each block of keys at another query block (+10 %).
 //
 // Parity: the reference calls a closed vendor flash backward (reference torch_musa/csrc/aten/ops/attention/mudnn/SDP.cpp:678-845).

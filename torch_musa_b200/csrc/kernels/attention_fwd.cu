@@ -48,9 +48,10 @@ struct AttnParams {
 // clock, and writing P there, fencing the async proxy and reading it back stood in the middle of the chain S -> softmax ->
 // P V.  One barrier per tile says "all products of this tile so far are done" (S of block j and, before it, P V of block
 // j - 1), so the softmax may overwrite S with P and rescale O without another wait.  What bounds the kernel now is that
-// chain: per block of 128 keys about 2700 clocks of softmax (two warpgroups share the special-function unit: 2048 clocks of
-// exponentials for both), 1050 of products and 500 of hand-over, while the tensor core has 2100 clocks of work for both
-// tiles.  Measured at 32 heads x 4096 x 128 bf16, before -> after: causal 174 -> 139 us (990 TFLOP/s), full 300 -> 255 us;
+// chain: per block of 128 keys an SM spends 3900 clocks on both tiles, the starts and ends of its CTAs included; the tensor core
+// is busy for 2050 of them (its counter: 50 %) and the special-function units, which the two warpgroups share, for 2050 too (52 %):
+// the softmax of a tile, its products and the hand-over follow one another, and two tiles are not enough to fill the gaps of
+// both.  Measured at 32 heads x 4096 x 128 bf16, before -> after: causal 174 -> 139 us (990 TFLOP/s), full 300 -> 255 us;
 // 32 heads x 16384 causal 1790 us (1230 TFLOP/s).  Tried and not kept: a quarter to a half of the exponentials as polynomials
 // on the FMA pipe (+2 to +10 % time), two warpgroups per tile (+11 %), S in halves of 64 keys issued ahead (+12 %: an N64
 // product is bound by reading A from shared memory).

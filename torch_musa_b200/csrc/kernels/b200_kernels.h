@@ -228,10 +228,10 @@ B200_API int b200_softmax_bwd(int dtype, void* dx, const void* dy, const void* y
 B200_API int b200_cross_entropy_fwd(int dtype, float* loss, float* lse, const void* logits, const int64_t* target,
                                     int64_t rows, int64_t cols, int64_t ignore_index, float label_smoothing,
                                     cudaStream_t stream);
-/* dlogits = (softmax - onehot) * grad_scale[row or scalar]; may run in place over logits */
 /* mean[0] = sum of loss over the rows / max(1, number of targets that are not ignore_index), count[0] = that number */
 B200_API int b200_cross_entropy_mean(float* mean, float* count, const float* loss, const int64_t* target, int64_t rows,
                                      int64_t ignore_index, cudaStream_t stream);
+/* dlogits = (softmax - onehot) * grad_scale[row or scalar]; may run in place over logits */
 B200_API int b200_cross_entropy_bwd(int dtype, void* dlogits, const void* logits, const float* lse,
                                     const int64_t* target, const float* grad_loss, int grad_is_scalar, float scale,
                                     int64_t rows, int64_t cols, int64_t ignore_index, float label_smoothing,

@@ -113,11 +113,11 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint6
 }
 // One lane of the (converged) warp.  The roles that issue MMAs or TMA copies run their loops with the whole warp and guard
 // only the asynchronous instructions with this predicate: inside an `if (lane == 0)` block the addresses and descriptors are
-// per-thread values, and moving them to the uniform registers that these instructions take costs more than the 64 clocks that
-// an M128 N128 K16 product runs for (measured: 75 clocks from one product to the next, 65 with the elected lane).  Before ->
-// after with nothing else changed: fp8 linear layer 4096 x 14336 x 4096 550 -> 494 us, grouped expert GEMMs in training
-// 9.00 -> 8.51 ms, 3x3 convolution with batch norm in training (with vector reductions in its weight gradient) 418 -> 405 us;
-// 0.7 to 1.2 % on the M256 N256 pair kernel, whose products are long enough to hide most of it.
+// per-thread values, and moving them to the uniform registers that these instructions take costs about as much as the 64 clocks
+// that an M128 N128 K16 product runs for.  Before -> after: fp8 linear layer 4096 x 14336 x 4096 550 -> 494 us with nothing else
+// changed; 3x3 convolution with batch norm in training, together with the vector reductions in its weight gradient, 421 -> 407 us;
+// grouped expert GEMMs in training 8.65 -> 8.39 ms, of which two runs of one side differ by 2 %; the M256 N256 pair kernel, whose
+// products are long enough to hide it, within 1 to 2 %.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(

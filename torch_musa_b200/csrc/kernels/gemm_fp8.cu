@@ -10,12 +10,12 @@
 // core works on the next block in the other accumulator.  The epilogue applies optional per-row / per-column factors (row-wise
 // and tensor-wise scaling are the special case of block factors 1) and the bias, and stores bf16 / fp16 / fp32; the ring fills
 // for the next tile meanwhile.
-// What bounds it: at FN = 256 a K block is 512 clocks of products and 96 KB through shared memory (48 KB in, 48 KB read: 768
-// clocks); the promotion takes 1100 to 1200 (512 clocks of multiply-adds and TMEM reads per scheduler with only two warps to
-// hide the latency of the reads), so it is the promotion.  4096 x 14336 x 4096: 545 us with one promotion warpgroup, FN = 128,
-// no persistence and row-wise 16-byte stores; 361 now (1330 TFLOP/s; products alone 290, promotion alone 306), of which the
-// staged epilogue is worth 20; 4096 x 11008 x 14336 1099 -> 811 (1595 TFLOP/s).  Four promotion warpgroups were slower
-// (626 us), a TMEM read per 32 columns too (372).
+// What bounds it: the promotion.  At FN = 256 an SM spends 1560 clocks on a K block, the epilogues included, of which the tensor
+// core is busy for 512 (its counter: 33 %) and shared memory for 768 (48 KB in, 48 KB read); the multiply-adds and TMEM reads of
+// the promotion take 512 issue clocks per scheduler, with only two warps there to hide the latency of the reads.  4096 x 14336 x
+// 4096: 545 us with one promotion warpgroup, FN = 128, no persistence and row-wise 16-byte stores; 361 now (1330 TFLOP/s; with
+// parts left out: products alone 290, promotion alone 306), of which the staged epilogue is worth 20; 4096 x 11008 x 14336 1099
+// -> 811 (1595 TFLOP/s).  Four promotion warpgroups were slower (626 us), a TMEM read per 32 columns too (372).
 // Every mbarrier wait is bounded.
 //
 // Parity: the reference forwards _scaled_mm to its vendor library (reference torch_musa/csrc/aten/ops/Matmul.cpp:670-681).
@@ -318,9 +318,10 @@ int launch_fp8(const b200_fp8_gemm_t* g, void* d, const void* a, const void* b, 
   B200K_LAUNCH_RET();
 }
 
-// Which tile: waves over the SMs times the time of a tile.  A 128 x 256 tile takes 1.6 times as long as a 128 x 128 one
-// (4096 x 14336 x 4096: 361 us in 13 waves; the narrow tile 494 in 25), so it wins as soon as the SMs have enough tiles of it;
-// few rows or columns go to the narrow one.
+// Which tile: waves over the SMs times the time of a tile.  A 128 x 256 tile takes 1.6 to 1.7 times as long as a 128 x 128 one
+// (4096 x 14336 x 4096: 356 us in 13 waves, the narrow tile 418 in 25; 3072 x 11008 x 4096: 196 in 7, 238 in 14), so it wins as
+// soon as the SMs have enough tiles of it: 1 wave against 2 21 / 24 us (640 x 4096 x 2048), 3 against 5 86 / 88 (2560 x 4096 x 4096), 4
+// against 7 112 / 119; 2 against 3 goes to the narrow one, 59 / 55 (1536 x 4096 x 4096), and 1 against 1 30 / 20.
 template <typename OutT>
 int launch_fp8_any(const b200_fp8_gemm_t* g, void* d, const void* a, const void* b, cudaStream_t stream) {
   const long long sms = gemm_sm_count(), tm = (g->m + FM - 1) / FM;
